@@ -1269,9 +1269,9 @@ def main():
                "overlapping the previous frame's fitter, weighted sum and TAA (same outputs bit for bit); "
                "single: one bmfr_denoise_frame_io call per frame, stages in stream order"}
     # noise table, block kernel, weighted sum + filtered accumulation, taa
-    # (fused); noise table, accumulate, fitter, weighted sum + filtered
-    # accumulation, taa (staged)
-    launches_per_frame = 4 if pipeline == B.PIPELINE_FUSED else 5
+    # (fused); accumulate, fitter, weighted sum + filtered accumulation, taa
+    # (staged)
+    launches_per_frame = 4
 
     # ---- per-stage profile (same workload, events between stages) ------------
     plan.enable_profiling(True)

@@ -313,7 +313,8 @@ cudaError_t launch_staged_step(bmfr_batch* b, const bmfr::BatchStepDesc& d, cuda
             used[w] = true;
         }
         load[w] += g.blocks;
-        if (e == cudaSuccess) e = bmfr::launch_noise_table(f, const_cast<float*>(fb.noise), ws);
+        if (e == cudaSuccess && bmfr::fitter_reads_noise_table(half_tmp, b->p.fp32_qr))
+            e = bmfr::launch_noise_table(f, const_cast<float*>(fb.noise), ws);
         if (e == cudaSuccess)
             e = bmfr::launch_accumulate_noisy(g, J.job.a, fb.prev_pix, fb.accept, fb.cur_n, fb.prev_n, fb.cur_p,
                                               fb.prev_p, fb.noisy_in, fb.noisy_acc_cur, fb.noisy_acc_prev, half_hist,

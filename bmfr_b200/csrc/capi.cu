@@ -523,7 +523,9 @@ int run_frame(bmfr_plan* plan, const float* albedo, const float* cur_n, const fl
         plan->downloaded[cur] = false;
     }
     mark(0);
-    if (e == cudaSuccess) e = bmfr::launch_noise_table(f, fs.noise_table, sa);
+    if (e == cudaSuccess && (plan->p.pipeline == BMFR_PIPELINE_FUSED ||
+                             bmfr::fitter_reads_noise_table(half_tmp, plan->p.fp32_qr)))
+        e = bmfr::launch_noise_table(f, fs.noise_table, sa);
     if (plan->p.pipeline == BMFR_PIPELINE_FUSED) {
         mark(1);
         bmfr::FusedBuffers fb;

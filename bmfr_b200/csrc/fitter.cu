@@ -1,6 +1,9 @@
-// fitter.cu — standalone fitter kernel (opencl/bmfr.cl:490-700).
+// fitter.cu — standalone fitter kernels (opencl/bmfr.cl:490-700).
 //
-// Persistent CTAs of 256 threads, as many as fit on the SMs.  Each CTA walks
+// k_fitter_rows16: the reference's arithmetic on binary16 tmp_data, groups of
+// 64 threads per block of the image (fit_rows16.cuh).
+//
+// k_fitter: everything else.  Persistent CTAs of 256 threads, as many as fit on the SMs.  Each CTA walks
 // blocks b = blockIdx.x, + gridDim.x, ...: a block's 13 x 1024 tmp_data
 // values arrive in shared memory by one TMA copy and move to registers, and
 // the copy of a later block is issued at once so that it overlaps the fit.
@@ -14,8 +17,8 @@
 // tile buffers, so the copy of the block after next is in flight while the
 // current one is fitted.  Float tmp_data uses a one-dimensional bulk copy.
 //
-// The feature-noise table of the frame is either formed by each CTA in its
-// shared memory (the drop-in entry point: no scratch memory, so calls on
+// There the feature-noise table of the frame is either formed by each CTA in
+// its shared memory (the drop-in entry point: no scratch memory, so calls on
 // different streams never share state) or read from a table that an earlier
 // kernel of the frame pipeline wrote to global memory (smaller CTAs, more of
 // them per SM).
@@ -28,6 +31,7 @@
 #include <type_traits>
 
 #include "fit_block.cuh"
+#include "fit_rows16.cuh"
 #include "kernels.h"
 #include "tma.cuh"
 
@@ -52,9 +56,10 @@ __device__ __forceinline__ uint32_t swizzled_half(uint32_t h) {
     return (r << 7) | ((((c >> 3) ^ r) & 7u) << 4) | ((c & 7u) << 1);
 }
 
-// METHOD (FitMethod): kFitReference rounds like the reference (a binary16
-// tile when tmp_data is binary16); the precision-form methods need binary16
-// tmp_data and work on a float tile.
+// METHOD (FitMethod): the precision-form methods on binary16 tmp_data, or the
+// reference's arithmetic on float tmp_data, which rounds nowhere in between;
+// both work on a float tile.  (Binary16 tmp_data with the reference's
+// arithmetic: k_fitter_rows16.)
 template <bool HALF_TMP, int METHOD, bool NOISE_GLOBAL>
 __global__ void __launch_bounds__(256, (HALF_TMP && METHOD != kFitHouseholder32) ? 3 : 2)
     k_fitter(int nblocks, int frame, NoiseConst nc, const void* __restrict__ tmp, const __grid_constant__ CUtensorMap tmap,
@@ -64,7 +69,7 @@ __global__ void __launch_bounds__(256, (HALF_TMP && METHOD != kFitHouseholder32)
     using Shared = FitterShared<HALF_TMP, NOISE_GLOBAL>;
     using TmpT = typename Shared::TmpT;
     constexpr int kStages = Shared::kStages;
-    constexpr bool ROUND = HALF_TMP && METHOD == kFitReference;
+    static_assert(HALF_TMP == (METHOD != kFitReference), "");
     extern __shared__ unsigned char smem_raw[];
     // The swizzled copy needs a 1024-byte aligned destination.
     Shared& S = *reinterpret_cast<Shared*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -103,7 +108,7 @@ __global__ void __launch_bounds__(256, (HALF_TMP && METHOD != kFitHouseholder32)
             }
             return;
         }
-        Tile<ROUND> t;
+        Tile<false> t;
         const TmpT* tile = S.tile[st];
         // Row k*16 + 4q + id/64 of the tile holds (k, q); its swizzle XOR
         // (low three row bits) does not depend on k.
@@ -117,13 +122,8 @@ __global__ void __launch_bounds__(256, (HALF_TMP && METHOD != kFitHouseholder32)
                 __half v[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) v[q] = *reinterpret_cast<const __half*>(base + qoff[q]);
-                if constexpr (ROUND) {
-                    t.h[k][0] = __halves2half2(v[0], v[1]);
-                    t.h[k][1] = __halves2half2(v[2], v[3]);
-                } else {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) t.set1(k, q, __half2float(v[q]));
-                }
+                for (int q = 0; q < 4; ++q) t.set1(k, q, __half2float(v[q]));
             } else {
                 const TmpT* col = tile + k * kBlockPixels + id;
 #pragma unroll
@@ -133,8 +133,77 @@ __global__ void __launch_bounds__(256, (HALF_TMP && METHOD != kFitHouseholder32)
         __syncthreads();   // the buffer is free again
         const int next = b + kStages * (int)gridDim.x;
         if (threadIdx.x == 0 && next < nblocks) issue(st, next);
-        fit_block<ROUND, METHOD>(t, noise, nc, S.sm, weights + (size_t)b * kFeatures * 3,
+        fit_block<false, METHOD>(t, noise, nc, S.sm, weights + (size_t)b * kFeatures * 3,
                                  mins_maxs + (size_t)b * kScaled * 2);
+    }
+}
+
+// The reference-arithmetic fit of binary16 tmp_data (fit_rows16.cuh): G groups
+// of S teams per CTA, one CTA per SM, each group walking blocks of its own.
+// The CTA forms the frame's noise table in its shared memory, which its groups
+// share; that saves the launch that wrote it to global memory (2.0-2.4 us).
+//
+// Bound by the FMA pipes: a packed operation takes two cycles on one of them
+// and a scalar one the same slot on either, ~21 k such cycles per warp and
+// block, of which a column's rank-one updates are half.  From four groups on
+// an SM the time hardly falls with more of them (8349 blocks: 365 us with
+// four, 318 with five, 295 with six).  One thread per work-item, 256 threads
+// per block and the columns in registers took 47 M warp instructions for the
+// 984 blocks of 1280x720, this takes 23 M: 69.5 -> 42.5 us; 2135 blocks
+// (1920x1080) 148 -> 87 us; 8349 (3840x2160) 543 -> 295 us.
+template <int G>
+struct FitterRows16Shared {
+    uint4 tile[G][kTileChunks];   // 1024-byte aligned, for the swizzled copy
+    Rows16Smem sm[G];
+    alignas(16) float noise[kNoiseTableFloats];
+};
+
+template <int S, int G>
+__global__ void __launch_bounds__(kTeam * S * G, 1)
+    k_fitter_rows16(int nblocks, int frame, NoiseConst nc, const __grid_constant__ CUtensorMap tmap,
+                    float* __restrict__ weights, float* __restrict__ mins_maxs, int* __restrict__ status) {
+    using Shared = FitterRows16Shared<G>;
+    extern __shared__ unsigned char smem_raw[];
+    Shared& sh = *reinterpret_cast<Shared*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    constexpr uint32_t kTileBytes = kBuffers * kBlockPixels * sizeof(__half);
+    constexpr int kThreads = kTeam * S;
+    const int group = threadIdx.x / kThreads, bar = 1 + group;
+    const int i = threadIdx.x % kTeam, team = threadIdx.x % kThreads / kTeam;
+    // The leader is not in the warp that ends a block with the back
+    // substitution, so the next block's copy runs beside it.
+    const bool leader = i == 32 && team == S - 1;
+    const int first = group * gridDim.x + blockIdx.x, stride = G * gridDim.x;
+    Rows16Smem& sm = sh.sm[group];
+    uint4* tile = sh.tile[group];
+    if (leader) {
+        mbar_init(&sm.bar, 1);
+        fence_barrier_init();
+        sm.status = 0;
+    }
+    for (int e = threadIdx.x; e < kNoiseTableFloats; e += kThreads * G) sh.noise[e] = noise16_value(e, frame);
+    const float4* noise = reinterpret_cast<const float4*>(sh.noise);
+    __syncthreads();
+    await_previous_kernel();
+
+    uint32_t phase = 0;
+    for (int b = first; b < nblocks; b += stride, phase ^= 1u) {
+        if (leader) {
+            // The tile was last touched by generic loads and stores.
+            fence_proxy_async();
+            mbar_arrive_expect_tx(&sm.bar, kTileBytes);
+            tensor_copy_2d_g2s(tile, &tmap, 0, b * kTileRows, &sm.bar);
+            if (!mbar_wait_bounded(&sm.bar, phase)) sm.status = kDevTimeout;
+        }
+        group_sync<S>(bar);
+        if (sm.status) {
+            if (leader) {
+                atomicExch(status, kDevTimeout);
+                mbar_wait_bounded(&sm.bar, phase);   // let the copy in flight land
+            }
+            return;
+        }
+        fit_rows16<S>(i, team, noise, nc, sm, tile, bar, weights + (size_t)b * kFeatures * 3,
+                      mins_maxs + (size_t)b * kScaled * 2);
     }
 }
 
@@ -195,6 +264,20 @@ static cudaError_t encode_tmp_map(const void* tmp, int nblocks, CUtensorMap* map
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+// Allows `smem` bytes per CTA and finds how many CTAs fit on the device.
+template <typename Kernel>
+static cudaError_t resident_ctas(Kernel kern, int threads, int smem, int dev, int* ctas) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0, sms = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+    if (e != cudaSuccess) return e;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    *ctas = (per_sm > 0 ? per_sm : 1) * sms;
+    return cudaSuccess;
+}
+
 template <bool HALF_TMP, int METHOD, bool NOISE_GLOBAL>
 static cudaError_t launch_fitter_t(int nblocks, int frame, NoiseConst nc, const void* tmp, float* weights,
                                    float* mins_maxs, const float* noise, int* status, cudaStream_t s) {
@@ -210,14 +293,8 @@ static cudaError_t launch_fitter_t(int nblocks, int frame, NoiseConst nc, const 
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     int cap = grid_cap[dev].load(std::memory_order_relaxed);
     if (cap == 0) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = resident_ctas(kern, kLocal, smem, dev, &cap);
         if (e != cudaSuccess) return e;
-        int per_sm = 0, sms = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLocal, smem);
-        if (e != cudaSuccess) return e;
-        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return e;
-        cap = (per_sm > 0 ? per_sm : 1) * sms;
         grid_cap[dev].store(cap, std::memory_order_relaxed);
     }
     const int grid = nblocks < cap ? nblocks : cap;
@@ -232,35 +309,80 @@ static cudaError_t launch_fitter_t(int nblocks, int frame, NoiseConst nc, const 
                           mins_maxs, noise, status);
 }
 
+template <int S, int G>
+static cudaError_t launch_rows16_t(int nblocks, int frame, NoiseConst nc, const CUtensorMap& map, float* weights,
+                                   float* mins_maxs, int* status, int dev, int sms, cudaStream_t s) {
+    auto kern = k_fitter_rows16<S, G>;
+    const int smem = (int)sizeof(FitterRows16Shared<G>) + 1024;   // + alignment slack
+    static std::atomic<bool> allowed[64];
+    if (!allowed[dev].load(std::memory_order_relaxed)) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        allowed[dev].store(true, std::memory_order_relaxed);
+    }
+    return launch_chained(kern, dim3(nblocks < sms ? nblocks : sms), dim3(kTeam * S * G), smem, s, nblocks, frame, nc,
+                          map, weights, mins_maxs, status);
+}
+
+static cudaError_t launch_rows16(int nblocks, int frame, NoiseConst nc, const void* tmp, float* weights,
+                                 float* mins_maxs, int* status, cudaStream_t s) {
+    if (nblocks <= 0) return cudaSuccess;
+    static std::atomic<int> sm_count[64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    int sms = sm_count[dev].load(std::memory_order_relaxed);
+    if (sms == 0) {
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        sm_count[dev].store(sms, std::memory_order_relaxed);
+    }
+    CUtensorMap map;
+    e = encode_tmp_map(tmp, nblocks, &map);
+    if (e != cudaSuccess) return e;
+    // Which shape for how many blocks per SM.  Up to three, one block's chain of
+    // ten columns is what takes the time, and several teams shorten it: 100
+    // blocks 17.3 us with four teams, 18.6 with two, 23.5 with one; 400 blocks
+    // 26.6 us with two, 29.8 with one.  Beyond, one team per block costs the
+    // fewest operations: 600 blocks 37.6 us against 44.2 with two teams.  A
+    // seventh group overloads two of the SM's four schedulers (3680 blocks:
+    // 157.4 us with seven, 156.8 with six; 2200: 109.1 against 97.2), so there
+    // are seven only where they take all blocks at once (986: 47.0 against
+    // 57.8 us).
+    const int per_sm = (nblocks + sms - 1) / sms;
+    if (per_sm <= 1) return launch_rows16_t<4, 1>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
+    if (per_sm <= 3) return launch_rows16_t<2, 3>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
+    if (per_sm == 7) return launch_rows16_t<1, 7>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
+    return launch_rows16_t<1, 6>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
+}
+
+bool fitter_reads_noise_table(bool half_tmp, int qr) { return !(half_tmp && qr == kFitReference); }
+
 cudaError_t launch_fitter(const Geometry& g, int frame, NoiseConst nc, const void* tmp, bool half_tmp,
                           int qr, float* weights, float* mins_maxs, const float* noise_table, int* status,
                           cudaStream_t s) {
     const int n = g.blocks;
     // The precision-form methods apply to binary16 tmp_data; float tmp_data
     // always takes the reference's arithmetic.
-    const int method = half_tmp ? qr : kFitReference;
+    if (half_tmp && qr == kFitReference) return launch_rows16(n, frame, nc, tmp, weights, mins_maxs, status, s);
     if (noise_table) {
         if (!half_tmp)
             return launch_fitter_t<false, kFitReference, true>(n, frame, nc, tmp, weights, mins_maxs, noise_table,
                                                                status, s);
-        if (method == kFitCholQR2)
+        if (qr == kFitCholQR2)
             return launch_fitter_t<true, kFitCholQR2, true>(n, frame, nc, tmp, weights, mins_maxs, noise_table,
                                                             status, s);
-        if (method == kFitHouseholder32)
-            return launch_fitter_t<true, kFitHouseholder32, true>(n, frame, nc, tmp, weights, mins_maxs,
-                                                                  noise_table, status, s);
-        return launch_fitter_t<true, kFitReference, true>(n, frame, nc, tmp, weights, mins_maxs, noise_table,
-                                                          status, s);
+        return launch_fitter_t<true, kFitHouseholder32, true>(n, frame, nc, tmp, weights, mins_maxs, noise_table,
+                                                              status, s);
     }
     if (!half_tmp)
         return launch_fitter_t<false, kFitReference, false>(n, frame, nc, tmp, weights, mins_maxs, nullptr, status,
                                                             s);
-    if (method == kFitCholQR2)
+    if (qr == kFitCholQR2)
         return launch_fitter_t<true, kFitCholQR2, false>(n, frame, nc, tmp, weights, mins_maxs, nullptr, status, s);
-    if (method == kFitHouseholder32)
-        return launch_fitter_t<true, kFitHouseholder32, false>(n, frame, nc, tmp, weights, mins_maxs, nullptr,
-                                                               status, s);
-    return launch_fitter_t<true, kFitReference, false>(n, frame, nc, tmp, weights, mins_maxs, nullptr, status, s);
+    return launch_fitter_t<true, kFitHouseholder32, false>(n, frame, nc, tmp, weights, mins_maxs, nullptr, status,
+                                                           s);
 }
 
 // ---------------------------------------------------------------------------
@@ -316,8 +438,10 @@ cudaError_t launch_fitter_static(const Geometry& g, int frame, NoiseConst nc, co
     if (e != cudaSuccess) return e;
     float* table = static_cast<float*>(base);
     int* status = reinterpret_cast<int*>(static_cast<unsigned char*>(base) + kStaticStatusOffset);
-    e = launch_noise_table(frame, table, s);   // rewrites the table the last call left
-    if (e != cudaSuccess) return e;
+    if (fitter_reads_noise_table(half_tmp, qr)) {
+        e = launch_noise_table(frame, table, s);   // rewrites the table the last call left
+        if (e != cudaSuccess) return e;
+    }
     return launch_fitter(g, frame, nc, tmp, half_tmp, qr, weights, mins_maxs, table, status, s);
 }
 
