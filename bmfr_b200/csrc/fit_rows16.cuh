@@ -161,11 +161,10 @@ __device__ __forceinline__ float dot_rows(const Rows& x, const Rows& u, float u0
 }
 
 // value + NOISE_AMOUNT*2*r rounded once, as add_noise_r2 gives it, for
-// binary16 values.  With |NOISE_AMOUNT| < 1 every binary16 value is a multiple
-// of the last place of p = RN(hi*r), so s - v is exact (Dekker's fast two-sum)
-// and one fused multiply-add gives what s misses of v + hi*r.
+// binary16 values and |NOISE_AMOUNT| < 1.  Every binary16 value is then a
+// multiple of the last place of p = RN(hi*r), so s - v is exact (Dekker's fast
+// two-sum) and one fused multiply-add gives what s misses of v + hi*r.
 __device__ __forceinline__ float2 add_noise_half2(float2 v, float2 r, NoiseConst c) {
-    if (!(fabsf(c.hi) < 2.0f)) return add_noise_r2(v, r, c);
     const float2 hi = dup2(c.hi);
     const float2 s = add2(v, rmul2(hi, r, c.neg_zero));
     const float2 left = fma2(hi, r, fma2(s, dup2(-1.0f), v));
@@ -174,6 +173,7 @@ __device__ __forceinline__ float2 add_noise_half2(float2 v, float2 r, NoiseConst
 
 // The column as float pairs with the first column's noise added to features
 // 1..9 (bmfr.cl:625-627).
+template <bool PLAIN>
 __device__ __forceinline__ void noised_rows(const Rows& x, int k, int i, const float4* __restrict__ noise,
                                             NoiseConst nc, float2 (&a)[kRowPairs]) {
 #pragma unroll
@@ -182,8 +182,9 @@ __device__ __forceinline__ void noised_rows(const Rows& x, int k, int i, const f
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const float4 r = noise[((k - 1) * 4 + q) * kTeam + i];
-        a[2 * q] = add_noise_half2(a[2 * q], make_float2(r.x, r.y), nc);
-        a[2 * q + 1] = add_noise_half2(a[2 * q + 1], make_float2(r.z, r.w), nc);
+        const float2 r01 = make_float2(r.x, r.y), r23 = make_float2(r.z, r.w);
+        a[2 * q] = PLAIN ? add_noise_half2(a[2 * q], r01, nc) : add_noise_r2(a[2 * q], r01, nc);
+        a[2 * q + 1] = PLAIN ? add_noise_half2(a[2 * q + 1], r23, nc) : add_noise_r2(a[2 * q + 1], r23, nc);
     }
 }
 
@@ -214,22 +215,22 @@ struct Reflection {
 // result.  An infinite or NaN dot product makes infinite or NaN numerators,
 // which are their own quotients.
 //
-// ONES: u is 1 but for row 0 (the first column is the constant feature), so
-// one quotient serves every other row.
-template <bool NOISE, bool ONES>
+// PLAIN: u is 1 but for row 0 (the first column is the constant feature), so
+// one quotient serves every other row; and the noise is below 1.
+template <bool NOISE, bool PLAIN>
 __device__ __forceinline__ Rows update_rows(const Rows& x, int k, int i, const Reflection& f, float dot,
                                             const float4* __restrict__ noise, NoiseConst nc) {
     Rows y;
     const float2 d2 = dup2(2.0f * dot);   // u * 2d rounds as 2u * d
     const float2 ny = dup2(f.ny), b2 = dup2(f.b);
     float2 a[kRowPairs];
-    if (NOISE) noised_rows(x, k, i, noise, nc, a);
+    if (NOISE) noised_rows<PLAIN>(x, k, i, noise, nc, a);
     auto subtract = [&](int p, float2 mq) {
         if (NOISE) y.h[p] = __float22half2_rn(add2(a[p], mq));
         else y.h[p] = __floats2half2_rn(add_f32_h(__low2half(x.h[p]), mq.x), add_f32_h(__high2half(x.h[p]), mq.y));
     };
     const bool finite = fabsf(dot) <= 0x1p100f;
-    if (ONES) {
+    if (PLAIN) {
         const float2 n = make_float2(i == 0 ? f.u[0].x * d2.x : d2.x, d2.x);
         const float2 mq = finite ? neg_quotient(n, ny, b2) : neg2(n);
         subtract(0, mq);
@@ -249,14 +250,16 @@ __device__ __forceinline__ Rows update_rows(const Rows& x, int k, int i, const R
 // One Householder column (bmfr.cl:549-655).  MODE 0: the first column, whose
 // dot products read features 1..9 with noise added; 1: the second, whose pass
 // applies the first column's update to the noised features; 2: the others.
-// ONES: column 0 is all ones.  f: the previous column's reflection on entry,
+// PLAIN: column 0 is all ones and the noise below 1, as in every frame the
+// pipeline makes; the other instance serves callers' own tmp_data and noise
+// (a test of the noise inside the loops cost 12 % of the time).  f: the previous column's reflection on entry,
 // this one's on return; out holds the dot products that go with it.
-template <int S, int MODE, bool ONES>
+template <int S, int MODE, bool PLAIN>
 __device__ __forceinline__ void qr_column16(int col, int i, int team, Reflection& f, const float4* __restrict__ noise,
                                             NoiseConst nc, Rows16Smem& sm, uint4* tile, int bar) {
     const int lane = threadIdx.x & 31, g = lane >> 3, j = lane & 7, warp = 2 * team + (i >> 5);
     Rows u = load_rows(tile, col, i);
-    if (MODE > 0) u = update_rows<MODE == 1, MODE == 1 && ONES>(u, col, i, f, sm.out[0], noise, nc);
+    if (MODE > 0) u = update_rows<MODE == 1, MODE == 1 && PLAIN>(u, col, i, f, sm.out[0], noise, nc);
     const float c0 = __low2float(u.h[0]);
     // Norm of rows >= col+1 (bmfr.cl:553-569); only row i can be above.
     if (team == 0) {
@@ -288,9 +291,9 @@ __device__ __forceinline__ void qr_column16(int col, int i, int team, Reflection
         for (int n = 0; n < N; ++n) {
             if (MODE == 0) {
                 float2 a[kRowPairs];
-                noised_rows(x[n], k + n * S, i, noise, nc, a);
+                noised_rows<PLAIN>(x[n], k + n * S, i, noise, nc, a);
                 float2 s01, s23;
-                if (ONES) {
+                if (PLAIN) {
                     if (i == 0) a[0].x = __fmul_rn(a[0].x, u0);
                     s01 = add2(dup2(0.0f), a[0]);
                     s23 = add2(dup2(0.0f), a[1]);
@@ -315,7 +318,7 @@ __device__ __forceinline__ void qr_column16(int col, int i, int team, Reflection
                 }
                 s[n] = s01.x + ((s01.y + s23.x) + s23.y);
             } else {
-                x[n] = update_rows<MODE == 1, MODE == 1 && ONES>(x[n], k + n * S, i, f, sm.out[k + n * S - col], noise, nc);
+                x[n] = update_rows<MODE == 1, MODE == 1 && PLAIN>(x[n], k + n * S, i, f, sm.out[k + n * S - col], noise, nc);
                 s[n] = dot_rows(x[n], u, u0, row0);
             }
         }
@@ -493,7 +496,7 @@ __device__ __forceinline__ void fit_rows16(int i, int team, const float4* __rest
     group_sync<S>(bar);
 
     Reflection f;
-    if (sm.ones[0] && sm.ones[1]) {
+    if (sm.ones[0] && sm.ones[1] && fabsf(nc.hi) < 2.0f) {
         qr_column16<S, 0, true>(0, i, team, f, noise, nc, sm, tile, bar);
         qr_column16<S, 1, true>(1, i, team, f, noise, nc, sm, tile, bar);
     } else {
