@@ -76,6 +76,18 @@ struct NoiseConst {
 __device__ __forceinline__ float fmin_cl(float x, float y) { return (y < x || x != x) ? y : x; }
 __device__ __forceinline__ float fmax_cl(float x, float y) { return (x < y || x != x) ? y : x; }
 
+// Minimum and maximum of three in one operation; NaN operands are skipped.
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 // mirror (bmfr.cl:209-216): valid for indices at most one size out of range.
 __device__ __forceinline__ int mirror(int i, int n) {
     if (i < 0) return -i - 1;
@@ -103,6 +115,37 @@ __device__ __forceinline__ int floor_to_int(float v) {
     if (f < -1073741824.0f) return -(1 << 30);
     if (f > 1073741824.0f) return 1 << 30;
     return (int)f;
+}
+
+// convert_int_rtn for indices that are tested against an image before use:
+// saturates, and NaN maps to INT_MIN.  i and i + 1 (in unsigned arithmetic)
+// lie outside every image wherever the position does.
+__device__ __forceinline__ int floor_index(float v) {
+    const int i = __float2int_rd(v);
+    return v == v ? i : (int)0x80000000;
+}
+
+// Quotients of several numerators by one divisor, each correctly rounded: the
+// divisor's correctly rounded reciprocal and Markstein's correction
+// (q = a*y; r = fma(-q, d, a); q' = fma(r, y, q); negated here, so that zero
+// quotients keep their sign).  `most`: the largest magnitude among the
+// numerators.  A numerator below 2^-100 may round one place off (its residual
+// is no longer exact); every caller adds the quotient to, or compares it with,
+// a value of ordinary size.
+__device__ __forceinline__ bool divides_fast(float d, float most) {
+    const float m = fabsf(d);
+    return m >= 0x1p-60f && m <= 0x1p60f && most <= 0x1p60f;
+}
+__device__ __forceinline__ float quotient(float a, float ny, float d) {
+    const float nq = a * ny;
+    return -__fmaf_rn(__fmaf_rn(nq, d, a), ny, nq);
+}
+__device__ __forceinline__ float3 divide3(float3 a, float d) {
+    if (divides_fast(d, fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)))) {
+        const float ny = -__frcp_rn(d);
+        return make_float3(quotient(a.x, ny, d), quotient(a.y, ny, d), quotient(a.z, ny, d));
+    }
+    return make_float3(a.x / d, a.y / d, a.z / d);
 }
 
 // random() (bmfr.cl:162-171): a 32-bit integer hash mapped to [0, 1].
@@ -145,6 +188,16 @@ __device__ __forceinline__ float scale(float v, float mn, float mx) {
 
 __device__ __forceinline__ float round_half(float v) {
     return __half2float(__float2half_rn(v));
+}
+
+// Two tmp_data values as binary16 (bmfr.cl:255-265, 468-475): clamped to the
+// largest finite value, NaN as 0.
+__device__ __forceinline__ __half2 pack_features(float a, float b) {
+    uint32_t v;
+    asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(b), "f"(a));
+    const __half2 h = *reinterpret_cast<__half2*>(&v);
+    v &= __heq2_mask(h, h);
+    return *reinterpret_cast<__half2*>(&v);
 }
 
 // Store of one tmp_data value, binary16 or float32 (bmfr.cl:255-265, 468-475).

@@ -3,8 +3,6 @@
 // expression keeps the reference's operation order.
 #pragma once
 
-#include <type_traits>
-
 #include "common.cuh"
 
 namespace bmfr {
@@ -23,13 +21,13 @@ struct AccumResult {
 
 // Reprojection, 4-tap history gather and blend of one pixel
 // (bmfr.cl:319-445).  `cur` is the pixel's colour before blending.
-// PREFETCH: the previous positions and normals of all in-image taps are
-// loaded before any tap is tested, so their latencies overlap (more
-// registers); the tests and the blend keep the reference's order either
-// way.  Measured on the float-history pipeline at 1280x720: 159.1 -> 156.2 us
-// per frame, and 184.7 -> 170.2 us in the fused block kernel; with binary16
-// histories it lost (1080p 218.4 -> 220.4 us), so it is off there.
-template <typename HistT, bool PREFETCH = std::is_same<HistT, float>::value>
+// The previous positions and normals of all in-image taps are loaded before
+// any tap is tested, so their latencies overlap; the tests and the blend keep
+// the reference's order.  Measured (accumulation by events, us, loaded where
+// tested / before): 1920x1080 with binary16 histories 72.6 / 63.0, 1280x720
+// 39.7 / 34.1; without it the float-history block kernel took 184.7 against
+// 170.2.
+template <typename HistT>
 __device__ __forceinline__ AccumResult accumulate_core(
     const Geometry& g, const AccumArgs& a, int px, int py, float3 wp, float3 nrm, float3 cur,
     const float* __restrict__ prev_n, const float* __restrict__ prev_p,
@@ -46,68 +44,92 @@ __device__ __forceinline__ AccumResult accumulate_core(
         float uvx = ((m[0] * wp.x + m[4] * wp.y) + m[8] * wp.z) + m[12] * 1.0f;
         float uvy = ((m[1] * wp.x + m[5] * wp.y) + m[9] * wp.z) + m[13] * 1.0f;
         const float w = ((m[3] * wp.x + m[7] * wp.y) + m[11] * wp.z) + m[15] * 1.0f;
-        uvx = uvx / w;
-        uvy = uvy / w;
+        if (divides_fast(w, fmaxf(fabsf(uvx), fabsf(uvy)))) {
+            const float ny = -__frcp_rn(w);
+            uvx = quotient(uvx, ny, w);
+            uvy = quotient(uvy, ny, w);
+        } else {
+            uvx = uvx / w;
+            uvy = uvy / w;
+        }
         uvx = (uvx + 1.0f) / 2.0f;
         uvy = (uvy + 1.0f) / 2.0f;
         r.ppx = uvx * (float)g.W - a.off_x;
         r.ppy = uvy * (float)g.H - (1.0f - a.off_y);
-        const int ix = floor_to_int(r.ppx), iy = floor_to_int(r.ppy);
+        const int ix = floor_index(r.ppx), iy = floor_index(r.ppy);
         const float fx = r.ppx - (float)ix, fy = r.ppy - (float)iy;
         const float ofx = 1.0f - fx, ofy = 1.0f - fy;
         const float wts[4] = {ofx * ofy, fx * ofy, ofx * fy, fx * fy};
-        float total = 0.0f;
+        const unsigned W = g.W, H = g.H;
+        const bool col[2] = {(unsigned)ix < W, (unsigned)ix + 1u < W};
+        const bool row[2] = {(unsigned)iy < H, (unsigned)iy + 1u < H};
+        // The taps of a row lie side by side: one address per row and buffer.
+        const int s0 = (int)((unsigned)iy * W + (unsigned)ix), s1 = (int)((unsigned)s0 + W);
+        const float* const p_row[2] = {prev_p + 3 * (ptrdiff_t)s0, prev_p + 3 * (ptrdiff_t)s1};
+        const float* const n_row[2] = {prev_n + 3 * (ptrdiff_t)s0, prev_n + 3 * (ptrdiff_t)s1};
+        const HistT* const c_row[2] = {prev_noisy + 3 * (ptrdiff_t)s0, prev_noisy + 3 * (ptrdiff_t)s1};
+        const uint8_t* const spp_row[2] = {prev_spp + s0, prev_spp + s1};
         float3 tp[4], tn[4];
-        int ts[4];
+        bool in[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int sx = ix + (i & 1), sy = iy + (i >> 1);
-            ts[i] = (sx >= 0 && sy >= 0 && sx < g.W && sy < g.H) ? sy * g.W + sx : -1;
-            if (PREFETCH && ts[i] >= 0) {
-                tp[i] = load3(prev_p, ts[i]);
-                tn[i] = load3(prev_n, ts[i]);
+            in[i] = col[i & 1] && row[i >> 1];
+            tp[i] = tn[i] = make_float3(0.f, 0.f, 0.f);
+            if (in[i]) {
+                tp[i] = load3(p_row[i >> 1], i & 1);
+                tn[i] = load3(n_row[i >> 1], i & 1);
             }
         }
+        float wt[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            if (ts[i] >= 0) {
-                const int s = ts[i];
-                const float3 pp = PREFETCH ? tp[i] : load3(prev_p, s);
-                const float dx = pp.x - wp.x, dy = pp.y - wp.y, dz = pp.z - wp.z;
-                if ((dx * dx + dy * dy) + dz * dz < a.pos_lim2) {
-                    const float3 pn = PREFETCH ? tn[i] : load3(prev_n, s);
-                    const float ex = pn.x - nrm.x, ey = pn.y - nrm.y, ez = pn.z - nrm.z;
-                    if ((ex * ex + ey * ey) + ez * ez < a.nrm_lim2) {
-                        r.accept |= (uint8_t)(1 << i);
-                        sample_spp = sample_spp + wts[i] * (float)prev_spp[s];
-                        const float3 pc = hist_load(prev_noisy, s);
-                        prev.x = prev.x + wts[i] * pc.x;
-                        prev.y = prev.y + wts[i] * pc.y;
-                        prev.z = prev.z + wts[i] * pc.z;
-                        total = total + wts[i];
-                    }
-                }
+            const float dx = tp[i].x - wp.x, dy = tp[i].y - wp.y, dz = tp[i].z - wp.z;
+            const float ex = tn[i].x - nrm.x, ey = tn[i].y - nrm.y, ez = tn[i].z - nrm.z;
+            in[i] = in[i] && (dx * dx + dy * dy) + dz * dz < a.pos_lim2 && (ex * ex + ey * ey) + ez * ez < a.nrm_lim2;
+            wt[i] = in[i] ? wts[i] : 0.0f;
+            if (in[i]) r.accept |= (uint8_t)(1 << i);
+        }
+        // The accepted taps' histories in one batch; the others add zeros,
+        // which change no sum.
+        float3 pc[4];
+        float ps[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            pc[i] = make_float3(0.f, 0.f, 0.f);
+            ps[i] = 0.0f;
+            if (in[i]) {
+                ps[i] = (float)spp_row[i >> 1][i & 1];
+                pc[i] = hist_load(c_row[i >> 1], i & 1);
             }
+        }
+        float total = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            sample_spp = sample_spp + wt[i] * ps[i];
+            prev.x = prev.x + wt[i] * pc[i].x;
+            prev.y = prev.y + wt[i] * pc[i].y;
+            prev.z = prev.z + wt[i] * pc[i].z;
+            total = total + wt[i];
         }
         if (total > 0.0f) {
-            prev.x = prev.x / total;
-            prev.y = prev.y / total;
-            prev.z = prev.z / total;
-            sample_spp = sample_spp / total;
-            alpha = 1.0f / (sample_spp + 1.0f);
-            alpha = fmax_cl(alpha, a.blend_alpha);
+            if (divides_fast(total, fmaxf(fmaxf(fabsf(prev.x), fabsf(prev.y)), fmaxf(fabsf(prev.z), sample_spp)))) {
+                const float ny = -__frcp_rn(total);
+                prev.x = quotient(prev.x, ny, total);
+                prev.y = quotient(prev.y, ny, total);
+                prev.z = quotient(prev.z, ny, total);
+                sample_spp = quotient(sample_spp, ny, total);
+            } else {
+                prev.x = prev.x / total;
+                prev.y = prev.y / total;
+                prev.z = prev.z / total;
+                sample_spp = sample_spp / total;
+            }
+            alpha = fmaxf(__frcp_rn(sample_spp + 1.0f), a.blend_alpha);
         }
     }
+    // convert_uchar_sat_rte(sample_spp) + 1, saturated (bmfr.cl:424-436).
     r.spp = 1;
-    if (alpha < 1.0f) {
-        if (sample_spp > 254.0f) {
-            r.spp = 255;
-        } else {
-            float q = rintf(sample_spp);
-            q = q < 0.f ? 0.f : (q > 255.f ? 255.f : q);
-            r.spp = (uint8_t)((int)q + 1);
-        }
-    }
+    if (alpha < 1.0f) r.spp = sample_spp > 254.0f ? 255 : (uint8_t)(__float2int_rn(sample_spp) + 1);
     const float om = 1.0f - alpha;
     r.color = make_float3(alpha * cur.x + om * prev.x, alpha * cur.y + om * prev.y,
                           alpha * cur.z + om * prev.z);
@@ -122,8 +144,19 @@ __device__ __forceinline__ void store_tmp_row(const Geometry& g, void* tmp, bool
     const size_t base = (size_t)(yb * g.MWb + xb) * kBuffers * kBlockPixels + (size_t)(yin * 32 + xin);
     const float f[kBuffers] = {1.0f, nrm.x, nrm.y, nrm.z, wp.x, wp.y, wp.z,
                                wp.x * wp.x, wp.y * wp.y, wp.z * wp.z, c.x, c.y, c.z};
+    if (half_tmp) {
+        __half* t = static_cast<__half*>(tmp) + base;
+        t[0] = __float2half_rn(1.0f);
 #pragma unroll
-    for (int k = 0; k < kBuffers; ++k) store_feature(tmp, base + (size_t)k * kBlockPixels, f[k], half_tmp);
+        for (int k = 1; k < kBuffers; k += 2) {
+            const __half2 h = pack_features(f[k], f[k + 1]);
+            t[k * kBlockPixels] = __low2half(h);
+            t[(k + 1) * kBlockPixels] = __high2half(h);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < kBuffers; ++k) store_feature(tmp, base + (size_t)k * kBlockPixels, f[k], false);
+    }
 }
 
 // accumulate_noisy_data of margin pixel (gx, gy) (bmfr.cl:310-484), out of
@@ -182,6 +215,51 @@ __device__ __forceinline__ float3 weighted_sum_px(float3 wp, float3 n, const flo
     return c;
 }
 
+// A block's weights and feature bounds as a CTA whose pixels all lie in the
+// block keeps them in shared memory: the divisions by the bounds' range need
+// one reciprocal per block.
+struct BlockFit {
+    float w[kFeatures * 3 + 2];
+    float mn[kScaled], d[kScaled], ny[kScaled];   // minimum, range, -RN(1/range)
+};
+
+// Filled by threads t = 0..63 of the CTA; a barrier follows.
+__device__ __forceinline__ void prepare_block_fit(BlockFit& f, const float* __restrict__ weights,
+                                                  const float* __restrict__ mins_maxs, int block, int t) {
+    if (t < kFeatures * 3) f.w[t] = weights[(size_t)block * kFeatures * 3 + t];
+    if (t >= 32 && t < 32 + kScaled) {
+        const float* mm = mins_maxs + (size_t)block * kScaled * 2 + 2 * (t - 32);
+        const float d = mm[1] - mm[0];
+        f.mn[t - 32] = mm[0];
+        f.d[t - 32] = d;
+        f.ny[t - 32] = -__frcp_rn(d);
+    }
+}
+
+// weighted_sum_px from a prepared block.  A quotient whose numerator is below
+// 2^-100 may round one place off; its product is added to a sum.
+__device__ __forceinline__ float3 weighted_sum_block(float3 wp, float3 n, const BlockFit& b) {
+    float v[kFeatures] = {1.0f, n.x, n.y, n.z, wp.x, wp.y, wp.z, wp.x * wp.x, wp.y * wp.y, wp.z * wp.z};
+#pragma unroll
+    for (int k = 0; k < kScaled; ++k) {
+        const float a = v[kNotScaled + k] - b.mn[k], d = b.d[k];
+        v[kNotScaled + k] = a;
+        if (fabsf(d) > 1.0f)   // the same for the whole CTA
+            v[kNotScaled + k] = divides_fast(d, fabsf(a)) ? quotient(a, b.ny[k], d) : a / d;
+    }
+    float3 c = make_float3(0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < kFeatures; ++k) {
+        c.x = c.x + b.w[3 * k] * v[k];
+        c.y = c.y + b.w[3 * k + 1] * v[k];
+        c.z = c.z + b.w[3 * k + 2] * v[k];
+    }
+    c.x = c.x < 0.f ? 0.f : c.x;
+    c.y = c.y < 0.f ? 0.f : c.y;
+    c.z = c.z < 0.f ? 0.f : c.z;
+    return c;
+}
+
 // accumulate_filtered_data body (bmfr.cl:778-856); returns the accumulated
 // colour and writes the tone-mapped one through `tm`.
 // Tone map: clamp(powr(max(0, albedo * acc), 0.454545), 0, 1) (bmfr.cl:853-854).
@@ -190,9 +268,9 @@ __device__ __forceinline__ float3 weighted_sum_px(float3 wp, float3 n, const flo
 // negligible absolute error below that (the OpenCL powr it stands for may
 // be 16 ulp off); several times cheaper than powf.
 __device__ __forceinline__ float tonemap1(float albedo, float acc) {
-    const float x = fmax_cl(0.0f, albedo * acc);
+    const float x = fmaxf(0.0f, albedo * acc);
     const float t = x > 0.0f ? exp2f(0.454545f * __log2f(x)) : 0.0f;
-    return fmin_cl(fmax_cl(t, 0.0f), 1.0f);
+    return fminf(t, 1.0f);
 }
 
 template <typename HistT>
@@ -203,27 +281,32 @@ __device__ __forceinline__ float3 accumulate_filtered_px(const Geometry& g, int 
     float3 prev = make_float3(0.f, 0.f, 0.f);
     float alpha = 1.0f;
     if (frame > 0 && acc > 0) {
-        const int ix = floor_to_int(pp.x), iy = floor_to_int(pp.y);
+        const int ix = floor_index(pp.x), iy = floor_index(pp.y);
         const float fx = pp.x - (float)ix, fy = pp.y - (float)iy;
         const float ofx = 1.0f - fx, ofy = 1.0f - fy;
         const float wts[4] = {ofx * ofy, fx * ofy, ofx * fy, fx * fy};
+        const int s0 = (int)((unsigned)iy * (unsigned)g.W + (unsigned)ix);
+        const HistT* const c_row[2] = {acc_prev + 3 * (ptrdiff_t)s0,
+                                       acc_prev + 3 * (ptrdiff_t)(int)((unsigned)s0 + (unsigned)g.W)};
+        // The accepted taps in one batch of loads; the others add zeros.
+        float3 c[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            c[i] = make_float3(0.f, 0.f, 0.f);
+            if (acc & (1 << i)) c[i] = hist_load(c_row[i >> 1], i & 1);
+        }
         float total = 0.0f;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            if (acc & (1 << i)) {
-                total = total + wts[i];
-                const float3 c = hist_load(acc_prev, (iy + (i >> 1)) * g.W + ix + (i & 1));
-                prev.x = prev.x + wts[i] * c.x;
-                prev.y = prev.y + wts[i] * c.y;
-                prev.z = prev.z + wts[i] * c.z;
-            }
+            const float w = acc & (1 << i) ? wts[i] : 0.0f;
+            total = total + w;
+            prev.x = prev.x + w * c[i].x;
+            prev.y = prev.y + w * c[i].y;
+            prev.z = prev.z + w * c[i].z;
         }
         if (total > 0.0f) {
-            alpha = 1.0f / (float)spp;
-            alpha = fmax_cl(alpha, second_alpha);
-            prev.x = prev.x / total;
-            prev.y = prev.y / total;
-            prev.z = prev.z / total;
+            alpha = fmaxf(__frcp_rn((float)spp), second_alpha);
+            prev = divide3(prev, total);
         }
     }
     const float om = 1.0f - alpha;
@@ -278,16 +361,18 @@ __device__ __forceinline__ void wsacc_px(const Geometry& g, int frame, float sec
 }
 
 // taa body (bmfr.cl:873-973).
-// YCoCg of one colour, unnormalised (bmfr.cl:184-198).
+// YCoCg of one colour, unnormalised (bmfr.cl:184-198).  The products by 2 are
+// exact, so each rounds as the reference's multiply and add.
 __device__ __forceinline__ void rgb_to_ycocg(float3 s, float (&ycc)[3]) {
-    ycc[0] = (s.x * 1.0f + s.y * 2.0f) + s.z * 1.0f;
-    ycc[1] = (s.x * 2.0f + s.y * 0.0f) + s.z * -2.0f;
-    ycc[2] = (s.x * -1.0f + s.y * 2.0f) + s.z * -1.0f;
+    ycc[0] = __fmaf_rn(2.0f, s.y, s.x) + s.z;
+    ycc[1] = __fmaf_rn(-2.0f, s.z, __fmaf_rn(0.0f, s.y, s.x + s.x));
+    ycc[2] = __fmaf_rn(2.0f, s.y, -s.x) - s.z;
 }
 
-// The second half of taa (bmfr.cl:904-973) for pixel (px, py) whose
-// tonemapped colour is `mine`, given the YCoCg bounds of its 3x3 box and
-// its cross: history bilinear, clamp, blend.
+// The second half of taa (bmfr.cl:904-973) for a pixel whose tonemapped
+// colour is `mine` and whose history position pp, with ix, iy its floor, has a
+// tap in the image, given the YCoCg bounds of its 3x3 box and its cross:
+// history bilinear, clamp, blend.
 template <typename HistT>
 __device__ __forceinline__ float3 taa_finish(const Geometry& g, float taa_alpha, float2 pp, int ix, int iy,
                                              float3 mine, const float (&mnb)[3], const float (&mxb)[3],
@@ -297,24 +382,28 @@ __device__ __forceinline__ float3 taa_finish(const Geometry& g, float taa_alpha,
     float total = 0.0f;
     const float fx = pp.x - (float)ix, fy = pp.y - (float)iy;
     const float ofx = 1.0f - fx, ofy = 1.0f - fy;
-    auto tap = [&](int sx, int sy, float w) {
-        const float3 s = hist_load(prev_frame, sy * g.W + sx);
-        prev.x = prev.x + w * s.x;
-        prev.y = prev.y + w * s.y;
-        prev.z = prev.z + w * s.z;
+    const HistT* const row0 = prev_frame + 3 * (ptrdiff_t)(iy * g.W + ix);
+    const HistT* const row1 = row0 + 3 * (ptrdiff_t)g.W;
+    // The taps in the image in one batch of loads; the others add zeros.
+    const float wts[4] = {ofx * ofy, fx * ofy, ofx * fy, fx * fy};
+    const bool col[2] = {ix >= 0, ix < g.W - 1}, row[2] = {iy >= 0, iy < g.H - 1};
+    float3 s[4];
+    bool in[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        in[i] = col[i & 1] && row[i >> 1];
+        s[i] = make_float3(0.f, 0.f, 0.f);
+        if (in[i]) s[i] = hist_load(i >> 1 ? row1 : row0, i & 1);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float w = in[i] ? wts[i] : 0.0f;
+        prev.x = prev.x + w * s[i].x;
+        prev.y = prev.y + w * s[i].y;
+        prev.z = prev.z + w * s[i].z;
         total = total + w;
-    };
-    if (iy >= 0) {
-        if (ix >= 0) tap(ix, iy, ofx * ofy);
-        if (ix < g.W - 1) tap(ix + 1, iy, fx * ofy);
     }
-    if (iy < g.H - 1) {
-        if (ix >= 0) tap(ix, iy + 1, ofx * fy);
-        if (ix < g.W - 1) tap(ix + 1, iy + 1, fx * fy);
-    }
-    prev.x = prev.x / total;
-    prev.y = prev.y / total;
-    prev.z = prev.z / total;
+    prev = divide3(prev, total);
     float pyc[3];
     rgb_to_ycocg(prev, pyc);
     float cl[3];
@@ -322,46 +411,18 @@ __device__ __forceinline__ float3 taa_finish(const Geometry& g, float taa_alpha,
     for (int c = 0; c < 3; ++c) {
         const float lo = (mnb[c] + mnc[c]) / 2.0f;
         const float hi = (mxb[c] + mxc[c]) / 2.0f;
-        cl[c] = fmin_cl(fmax_cl(pyc[c], lo), hi);
+        cl[c] = fminf(fmaxf(pyc[c], lo), hi);   // fmin/fmax: the bound where pyc is NaN
+        // A cross without a number has the bounds +inf and -inf.
+        if (mnc[c] != mnc[c]) cl[c] = -INFINITY;
     }
-    const float3 rgb = make_float3((cl[0] * 0.25f + cl[1] * 0.25f) + cl[2] * -0.25f,
-                                   (cl[0] * 0.25f + cl[1] * 0.0f) + cl[2] * 0.25f,
-                                   (cl[0] * 0.25f + cl[1] * -0.25f) + cl[2] * -0.25f);
+    // The products by 1/4 and 0 are exact (bmfr.cl:965-967).
+    const float a = cl[0] * 0.25f;
+    const float3 rgb = make_float3(__fmaf_rn(-0.25f, cl[2], __fmaf_rn(0.25f, cl[1], a)),
+                                   __fmaf_rn(0.25f, cl[2], __fmaf_rn(0.0f, cl[1], a)),
+                                   __fmaf_rn(-0.25f, cl[2], __fmaf_rn(-0.25f, cl[1], a)));
     const float om = 1.0f - taa_alpha;
     return make_float3(taa_alpha * mine.x + om * rgb.x, taa_alpha * mine.y + om * rgb.y,
                        taa_alpha * mine.z + om * rgb.z);
-}
-
-// taa (bmfr.cl:868-973) of pixel (px, py) whose tonemapped colour is `mine`;
-// nb(x, y, ycc) gives the YCoCg of the in-image neighbour (px+x, py+y).
-template <typename HistT, typename Nb>
-__device__ __forceinline__ float3 taa_core(const Geometry& g, int frame, float taa_alpha, int px, int py, float2 pp,
-                                           float3 mine, Nb&& nb, const HistT* __restrict__ prev_frame) {
-    const int ix = floor_to_int(pp.x), iy = floor_to_int(pp.y);
-    if (frame == 0 || ix < -1 || iy < -1 || ix >= g.W || iy >= g.H) return mine;
-    float mnb[3] = {INFINITY, INFINITY, INFINITY}, mnc[3] = {INFINITY, INFINITY, INFINITY};
-    float mxb[3] = {-INFINITY, -INFINITY, -INFINITY}, mxc[3] = {-INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-    for (int y = -1; y < 2; ++y) {
-#pragma unroll
-        for (int x = -1; x < 2; ++x) {
-            const int sx = px + x, sy = py + y;
-            if (sx >= 0 && sy >= 0 && sx < g.W && sy < g.H) {
-                float ycc[3];
-                nb(x, y, ycc);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    if (x == 0 || y == 0) {
-                        mnc[c] = fmin_cl(mnc[c], ycc[c]);
-                        mxc[c] = fmax_cl(mxc[c], ycc[c]);
-                    }
-                    mnb[c] = fmin_cl(mnb[c], ycc[c]);
-                    mxb[c] = fmax_cl(mxb[c], ycc[c]);
-                }
-            }
-        }
-    }
-    return taa_finish(g, taa_alpha, pp, ix, iy, mine, mnb, mxb, mnc, mxc, prev_frame);
 }
 
 // taa over a strip of R rows per thread.  A warp covers 30 image columns
@@ -370,10 +431,9 @@ __device__ __forceinline__ float3 taa_core(const Geometry& g, int frame, float t
 // rows with the halo), takes its left and right neighbours by shuffles, and
 // keeps a three-row window of horizontal minima and maxima, so a pixel's
 // nine neighbours cost about one load and one YCoCg conversion.  Neighbours
-// outside the image or NaN enter as +-inf, which the reference's fmin/fmax
-// ignore in the same way (bmfr.cl:884-902; fmin/fmax return the other
-// operand of a NaN), so the bounds equal the reference's up to the sign of a
-// zero bound.
+// outside the image enter as NaN, which minimum and maximum skip as the
+// reference's fmin/fmax do (bmfr.cl:884-902), so the bounds equal the
+// reference's up to the sign of a zero bound.
 template <int R, typename HistT>
 __device__ __forceinline__ void taa_strip(const Geometry& g, int frame, float taa_alpha, int x0, int y0,
                                           const float2* __restrict__ prev_pix, const float* __restrict__ new_frame,
@@ -383,8 +443,9 @@ __device__ __forceinline__ void taa_strip(const Geometry& g, int frame, float ta
     const int x = x0 - 1 + lane;
     const bool col_in = x >= 0 && x < g.W;
     const bool writer = lane >= 1 && lane <= 30 && col_in;
+    const float nan = __int_as_float(0x7fffffff);
     float3 rgb[3];
-    float cmn[3][3], cmx[3][3], hmn[3][3], hmx[3][3];   // [window row][channel]
+    float own[3][3], hmn[3][3], hmx[3][3];   // [window row][channel]
     // The strip's reprojected positions first: the history gather of each
     // row depends on them, and they depend on nothing here (1920x1080
     // frame 319.4 -> 315.2 us).
@@ -399,24 +460,17 @@ __device__ __forceinline__ void taa_strip(const Geometry& g, int frame, float ta
         const int k = r % 3;
         const int y = y0 - 1 + r;
         const bool in = col_in && y >= 0 && y < g.H;
-        const float3 s = in ? load3(new_frame, y * g.W + x) : make_float3(0.f, 0.f, 0.f);
+        const float3 s = in ? load3(new_frame, y * g.W + x) : make_float3(nan, nan, nan);
         rgb[k] = s;
-        float ycc[3];
-        rgb_to_ycocg(s, ycc);
+        rgb_to_ycocg(s, own[k]);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            // Out-of-image entries as NaN, which fminf/fmaxf skip (they
-            // return the other operand), so one shuffle each way serves both
-            // bounds; the pixel's own candidates turn a NaN into +-inf.
             // Lanes 0 and 31, the halo columns, take their own as a
             // neighbour and are not written.
-            const float v = in ? ycc[c] : __int_as_float(0x7fffffff);
+            const float v = own[k][c];
             const float vl = __shfl_up_sync(0xffffffffu, v, 1), vr = __shfl_down_sync(0xffffffffu, v, 1);
-            const float vmn = fminf(v, INFINITY), vmx = fmaxf(v, -INFINITY);
-            cmn[k][c] = vmn;
-            cmx[k][c] = vmx;
-            hmn[k][c] = fminf(fminf(vl, vmn), vr);
-            hmx[k][c] = fmaxf(fmaxf(vl, vmx), vr);
+            hmn[k][c] = min3(vl, v, vr);
+            hmx[k][c] = max3(vl, v, vr);
         }
         if (r >= 2) {
             const int up = (r - 2) % 3, mid = (r - 1) % 3, dn = k;
@@ -425,16 +479,16 @@ __device__ __forceinline__ void taa_strip(const Geometry& g, int frame, float ta
                 const int lp = py * g.W + x;
                 const float2 pp = ppre[r - 2];
                 const float3 mine = rgb[mid];
-                const int ix = floor_to_int(pp.x), iy = floor_to_int(pp.y);
+                const int ix = floor_index(pp.x), iy = floor_index(pp.y);
                 float3 out = mine;
-                if (!(frame == 0 || ix < -1 || iy < -1 || ix >= g.W || iy >= g.H)) {
+                if (frame > 0 && (unsigned)ix + 1u <= (unsigned)g.W && (unsigned)iy + 1u <= (unsigned)g.H) {
                     float mnb[3], mxb[3], mnc[3], mxc[3];
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        mnb[c] = fminf(fminf(hmn[up][c], hmn[mid][c]), hmn[dn][c]);
-                        mxb[c] = fmaxf(fmaxf(hmx[up][c], hmx[mid][c]), hmx[dn][c]);
-                        mnc[c] = fminf(fminf(cmn[up][c], hmn[mid][c]), cmn[dn][c]);
-                        mxc[c] = fmaxf(fmaxf(cmx[up][c], hmx[mid][c]), cmx[dn][c]);
+                        mnb[c] = min3(hmn[up][c], hmn[mid][c], hmn[dn][c]);
+                        mxb[c] = max3(hmx[up][c], hmx[mid][c], hmx[dn][c]);
+                        mnc[c] = min3(own[up][c], hmn[mid][c], own[dn][c]);
+                        mxc[c] = max3(own[up][c], hmx[mid][c], own[dn][c]);
                     }
                     out = taa_finish(g, taa_alpha, pp, ix, iy, mine, mnb, mxb, mnc, mxc, prev_frame);
                 }
@@ -444,19 +498,5 @@ __device__ __forceinline__ void taa_strip(const Geometry& g, int frame, float ta
         }
     }
 }
-
-// taa of one pixel, neighbours read from global memory.
-template <typename HistT>
-__device__ __forceinline__ float3 taa_px(const Geometry& g, int frame, float taa_alpha, int px, int py,
-                                         float2 pp, const float* __restrict__ new_frame,
-                                         const HistT* __restrict__ prev_frame) {
-    const float3 mine = load3(new_frame, py * g.W + px);
-    auto nb = [&](int x, int y, float (&ycc)[3]) {
-        const float3 s = (x == 0 && y == 0) ? mine : load3(new_frame, (py + y) * g.W + px + x);
-        rgb_to_ycocg(s, ycc);
-    };
-    return taa_core(g, frame, taa_alpha, px, py, pp, mine, nb, prev_frame);
-}
-
 
 }  // namespace bmfr

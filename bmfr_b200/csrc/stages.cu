@@ -22,8 +22,13 @@ namespace bmfr {
 //         wrote in pass 1 (in-place, second pass).
 // HistT: element type of the accumulated-colour history (noisy_out and
 // prev_noisy); in-place modes use float.
+//
+// Bound by the latency of its dependent gathers (position, then taps, then the
+// accepted taps' histories), so by warps in flight: CTAs of 128 threads, nine
+// per SM at 56 registers, against four of 256 at 58 (3840x2160 214 -> 201 us
+// by events, 1280x720 33.4 -> 31.2; ten at 48 registers spill: 203 and 31.5).
 template <int MODE, typename HistT>
-__global__ void __launch_bounds__(256) k_accumulate_noisy(
+__global__ void __launch_bounds__(128, 9) k_accumulate_noisy(
     Geometry g, AccumArgs a, float2* __restrict__ prev_pix, uint8_t* __restrict__ accept,
     const float* __restrict__ cur_n, const float* __restrict__ prev_n,
     const float* __restrict__ cur_p, const float* __restrict__ prev_p,
@@ -31,7 +36,7 @@ __global__ void __launch_bounds__(256) k_accumulate_noisy(
     const uint8_t* __restrict__ prev_spp, uint8_t* __restrict__ cur_spp, void* __restrict__ tmp) {
     await_previous_kernel();
     const int gx = blockIdx.x * 32 + threadIdx.x;
-    const int gy = blockIdx.y * 8 + threadIdx.y;
+    const int gy = blockIdx.y * 4 + threadIdx.y;
     if constexpr (MODE == 0) {
         accumulate_margin_px<HistT>(g, a, gx, gy, prev_pix, accept, cur_n, prev_n, cur_p, prev_p, noisy_in, noisy_out,
                                     prev_noisy, prev_spp, cur_spp, tmp);
@@ -66,18 +71,35 @@ __global__ void __launch_bounds__(256) k_accumulate_noisy(
 // weighted_sum, accumulate_filtered_data, taa
 // ---------------------------------------------------------------------------
 
+// The weighted sums run over the fitter's blocks, not over image tiles: a CTA
+// covers 8 rows of one block, so its weights and bounds come from shared
+// memory (42 loads per pixel otherwise) and a quotient by a feature's range
+// costs three operations.
+__device__ __forceinline__ bool block_pixel(const Geometry& g, int frame, int* px, int* py) {
+    const int2 bo = c_block_offsets[frame & 15];
+    *px = blockIdx.x * 32 + threadIdx.x - kBlockEdge / 2 + bo.x;
+    *py = blockIdx.y * 8 + threadIdx.y - kBlockEdge / 2 + bo.y;
+    return (unsigned)*px < (unsigned)g.W && (unsigned)*py < (unsigned)g.H;
+}
+
 __global__ void __launch_bounds__(256) k_weighted_sum(Geometry g, int frame,
                                                       const float* __restrict__ weights,
                                                       const float* __restrict__ mins_maxs,
                                                       float* __restrict__ out,
                                                       const float* __restrict__ cur_n,
                                                       const float* __restrict__ cur_p) {
-    const int px = blockIdx.x * 32 + threadIdx.x, py = blockIdx.y * 8 + threadIdx.y;
-    if (px >= g.W || py >= g.H) return;
+    __shared__ BlockFit fit;
+    prepare_block_fit(fit, weights, mins_maxs, (blockIdx.y >> 2) * g.MWb + blockIdx.x, threadIdx.y * 32 + threadIdx.x);
+    int px, py;
+    const bool in_image = block_pixel(g, frame, &px, &py);
     const int lp = py * g.W + px;
-    const int gi = pixel_block(g, frame, px, py);
-    store3(out, lp, weighted_sum_px(load3(cur_p, lp), load3(cur_n, lp), weights + (size_t)gi * kFeatures * 3,
-                                    mins_maxs + (size_t)gi * kScaled * 2));
+    float3 p, n;
+    if (in_image) {
+        p = load3(cur_p, lp);
+        n = load3(cur_n, lp);
+    }
+    __syncthreads();
+    if (in_image) store3(out, lp, weighted_sum_block(p, n, fit));
 }
 
 __global__ void __launch_bounds__(256) k_accumulate_filtered(
@@ -111,10 +133,33 @@ __global__ void __launch_bounds__(256) k_weighted_sum_accumulate(
     const uint8_t* __restrict__ cur_spp, const HistT* __restrict__ acc_prev,
     HistT* __restrict__ acc_cur) {
     await_previous_kernel();
-    const int px = blockIdx.x * 32 + threadIdx.x, py = blockIdx.y * 8 + threadIdx.y;
-    if (px >= g.W || py >= g.H) return;
-    wsacc_px<HistT>(g, frame, second_alpha, px, py, weights, mins_maxs, cur_n, cur_p, filtered, prev_pix, accept,
-                    albedo, tone_mapped, cur_spp, acc_prev, acc_cur);
+    __shared__ BlockFit fit;
+    prepare_block_fit(fit, weights, mins_maxs, (blockIdx.y >> 2) * g.MWb + blockIdx.x, threadIdx.y * 32 + threadIdx.x);
+    int px, py;
+    const bool in_image = block_pixel(g, frame, &px, &py);
+    const int lp = py * g.W + px;
+    float3 p, n;
+    float2 pp = make_float2(0.f, 0.f);
+    uint8_t acc = 0, spp = 1;
+    if (in_image) {
+        // Everything the history gather waits for is loaded before the barrier.
+        if (frame > 0) {
+            acc = accept[lp];
+            pp = prev_pix[lp];
+            spp = cur_spp[lp];
+        }
+        p = load3(cur_p, lp);
+        n = load3(cur_n, lp);
+    }
+    __syncthreads();
+    if (!in_image) return;
+    const float3 f = weighted_sum_block(p, n, fit);
+    float3 tm;
+    const float3 a3 = accumulate_filtered_px(g, frame, lp, f, pp, acc, spp, second_alpha, acc_prev, load3(albedo, lp),
+                                             &tm);
+    if (filtered) store3(filtered, lp, f);
+    hist_store(acc_cur, lp, a3);
+    store3(tone_mapped, lp, tm);
 }
 
 // Rows per warp strip: 2 rows (4 rows loaded with the halo) keep more warps
@@ -147,7 +192,7 @@ cudaError_t launch_accumulate_noisy(const Geometry& g, const AccumArgs& a, float
                                     const float* prev_p, const float* noisy_in, void* noisy_out,
                                     const void* prev_noisy, bool half_history, const uint8_t* prev_spp,
                                     uint8_t* cur_spp, void* tmp, cudaStream_t s) {
-    const dim3 grid = margin_grid(g), block(32, 8);
+    const dim3 grid(g.MW / 32, g.MH / 4), block(32, 4);
     if (half_history)
         return launch_chained(k_accumulate_noisy<0, __half>, grid, block, 0, s, g, a, prev_pix, accept, cur_n,
                               prev_n, cur_p, prev_p, noisy_in, (__half*)noisy_out, (const __half*)prev_noisy,
@@ -168,7 +213,7 @@ cudaError_t launch_accumulate_noisy(const Geometry& g, const AccumArgs& a, float
 
 cudaError_t launch_weighted_sum(const Geometry& g, int frame, const float* weights, const float* mins_maxs,
                                 float* out, const float* cur_n, const float* cur_p, cudaStream_t s) {
-    k_weighted_sum<<<image_grid(g), dim3(32, 8), 0, s>>>(g, frame, weights, mins_maxs, out, cur_n, cur_p);
+    k_weighted_sum<<<margin_grid(g), dim3(32, 8), 0, s>>>(g, frame, weights, mins_maxs, out, cur_n, cur_p);
     return cudaGetLastError();
 }
 
@@ -189,10 +234,10 @@ cudaError_t launch_weighted_sum_accumulate(const Geometry& g, int frame, float s
                                            const uint8_t* cur_spp, const void* acc_prev, void* acc_cur,
                                            bool half_history, cudaStream_t s) {
     if (half_history)
-        return launch_chained(k_weighted_sum_accumulate<__half>, image_grid(g), dim3(32, 8), 0, s, g, frame,
+        return launch_chained(k_weighted_sum_accumulate<__half>, margin_grid(g), dim3(32, 8), 0, s, g, frame,
                               second_alpha, weights, mins_maxs, cur_n, cur_p, filtered, prev_pix, accept, albedo,
                               tone_mapped, cur_spp, (const __half*)acc_prev, (__half*)acc_cur);
-    return launch_chained(k_weighted_sum_accumulate<float>, image_grid(g), dim3(32, 8), 0, s, g, frame, second_alpha,
+    return launch_chained(k_weighted_sum_accumulate<float>, margin_grid(g), dim3(32, 8), 0, s, g, frame, second_alpha,
                           weights, mins_maxs, cur_n, cur_p, filtered, prev_pix, accept, albedo, tone_mapped, cur_spp,
                           (const float*)acc_prev, (float*)acc_cur);
 }
