@@ -798,8 +798,8 @@ __device__ __forceinline__ void gram_finish(FitterSmem& sm) {
 // the Gram matrix (g[i], i <= j; zeros below) and stores its diagonal entry
 // in diag[j]; lanes 10..12 gather the colour column c = lane - 10 of the
 // second pass; other lanes zeros.
-template <bool PASS2>
-__device__ __forceinline__ void gram_columns(FitterSmem& sm, int lane, float (&g)[kFeatures]) {
+template <bool PASS2, typename Smem>
+__device__ __forceinline__ void gram_columns(Smem& sm, int lane, float (&g)[kFeatures]) {
 #pragma unroll
     for (int i = 0; i < kFeatures; ++i) {
         int e = -1;
@@ -842,6 +842,36 @@ __device__ __forceinline__ void chol_lanes(float (&g)[kFeatures], int lane, cons
         }
     }
     __syncwarp();
+}
+
+// The weights from the second factorisation, by the warp that made it: lane
+// j < 10 holds column j of R2, lanes 10..12 the colours' z; R1 in Rm.
+__device__ __forceinline__ void solve_weights(const float (&g)[kFeatures], int lane, const float (&Rm)[10][10],
+                                              const float* inv1, const float* inv2, float* __restrict__ weights_out) {
+    // R2 v = z in lanes 10..12 (R2(i, j) is lane j's g[i]) ...
+    float v[kFeatures];
+#pragma unroll
+    for (int ii = 0; ii < kFeatures; ++ii) {
+        const int i = kFeatures - 1 - ii;
+        float s = g[i];
+#pragma unroll
+        for (int j = i + 1; j < kFeatures; ++j) s = __fmaf_rn(-__shfl_sync(kFull, g[i], j), v[j], s);
+        v[i] = s * inv2[i];
+    }
+    // ... then R1 w = v.
+    float w[kFeatures];
+#pragma unroll
+    for (int ii = 0; ii < kFeatures; ++ii) {
+        const int i = kFeatures - 1 - ii;
+        float s = v[i];
+#pragma unroll
+        for (int j = i + 1; j < kFeatures; ++j) s = __fmaf_rn(-Rm[j][i], w[j], s);
+        w[i] = s * inv1[i];
+    }
+    if (lane >= kFeatures && lane < kFeatures + 3) {
+#pragma unroll
+        for (int k = 0; k < kFeatures; ++k) weights_out[3 * k + (lane - kFeatures)] = w[k];
+    }
 }
 
 // The fit of a scaled block (float tile, min/max already applied).
@@ -894,30 +924,7 @@ __device__ __forceinline__ void fit_columns_cqr2(Tile<false>& t, const float* __
         float g[kFeatures];
         gram_columns<true>(sm, lane, g);
         chol_lanes(g, lane, sm.diag, sm.inv2);
-        // R2 v = z in lanes 10..12 (R2(i, j) is lane j's g[i]) ...
-        float v[kFeatures];
-#pragma unroll
-        for (int ii = 0; ii < kFeatures; ++ii) {
-            const int i = kFeatures - 1 - ii;
-            float s = g[i];
-#pragma unroll
-            for (int j = i + 1; j < kFeatures; ++j) s = __fmaf_rn(-__shfl_sync(kFull, g[i], j), v[j], s);
-            v[i] = s * sm.inv2[i];
-        }
-        // ... then R1 w = v.
-        float w[kFeatures];
-#pragma unroll
-        for (int ii = 0; ii < kFeatures; ++ii) {
-            const int i = kFeatures - 1 - ii;
-            float s = v[i];
-#pragma unroll
-            for (int j = i + 1; j < kFeatures; ++j) s = __fmaf_rn(-sm.Rm[j][i], w[j], s);
-            w[i] = s * sm.inv1[i];
-        }
-        if (lane >= kFeatures && lane < kFeatures + 3) {
-#pragma unroll
-            for (int k = 0; k < kFeatures; ++k) weights_out[3 * k + (lane - kFeatures)] = w[k];
-        }
+        solve_weights(g, lane, sm.Rm, sm.inv1, sm.inv2, weights_out);
     }
     __syncthreads();
 }

@@ -1,7 +1,8 @@
 // fitter.cu — standalone fitter kernels (opencl/bmfr.cl:490-700).
 //
 // k_fitter_rows16: the reference's arithmetic on binary16 tmp_data, groups of
-// 64 threads per block of the image (fit_rows16.cuh).
+// 64 threads per block of the image (fit_rows16.cuh).  k_fitter_cqr2: the
+// precision form's CholeskyQR2, the same way (fit_cqr2.cuh).
 //
 // k_fitter: everything else.  Persistent CTAs of 256 threads, as many as fit on the SMs.  Each CTA walks
 // blocks b = blockIdx.x, + gridDim.x, ...: a block's 13 x 1024 tmp_data
@@ -31,6 +32,7 @@
 #include <type_traits>
 
 #include "fit_block.cuh"
+#include "fit_cqr2.cuh"
 #include "fit_rows16.cuh"
 #include "kernels.h"
 #include "tma.cuh"
@@ -56,12 +58,11 @@ __device__ __forceinline__ uint32_t swizzled_half(uint32_t h) {
     return (r << 7) | ((((c >> 3) ^ r) & 7u) << 4) | ((c & 7u) << 1);
 }
 
-// METHOD (FitMethod): the precision-form methods on binary16 tmp_data, or the
-// reference's arithmetic on float tmp_data, which rounds nowhere in between;
-// both work on a float tile.  (Binary16 tmp_data with the reference's
-// arithmetic: k_fitter_rows16.)
+// METHOD (FitMethod): the FP32 Householder sequence on binary16 tmp_data, or
+// the reference's arithmetic on float tmp_data, which rounds nowhere in
+// between; both work on a float tile.
 template <bool HALF_TMP, int METHOD, bool NOISE_GLOBAL>
-__global__ void __launch_bounds__(256, (HALF_TMP && METHOD != kFitHouseholder32) ? 3 : 2)
+__global__ void __launch_bounds__(256, 2)
     k_fitter(int nblocks, int frame, NoiseConst nc, const void* __restrict__ tmp, const __grid_constant__ CUtensorMap tmap,
              float* __restrict__ weights, float* __restrict__ mins_maxs, const float* __restrict__ noise_g,
              int* __restrict__ status) {
@@ -69,7 +70,7 @@ __global__ void __launch_bounds__(256, (HALF_TMP && METHOD != kFitHouseholder32)
     using Shared = FitterShared<HALF_TMP, NOISE_GLOBAL>;
     using TmpT = typename Shared::TmpT;
     constexpr int kStages = Shared::kStages;
-    static_assert(HALF_TMP == (METHOD != kFitReference), "");
+    static_assert(METHOD == (HALF_TMP ? kFitHouseholder32 : kFitReference), "");
     extern __shared__ unsigned char smem_raw[];
     // The swizzled copy needs a 1024-byte aligned destination.
     Shared& S = *reinterpret_cast<Shared*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -207,6 +208,69 @@ __global__ void __launch_bounds__(kTeam * S * G, 1)
     }
 }
 
+// The precision form's CholeskyQR2 fit (fit_cqr2.cuh): G groups of S teams per
+// CTA, one CTA per SM, as k_fitter_rows16.
+//
+// Bound by the FMA pipes (~2.4 k cycles of each scheduler per block: the
+// Gram entries' multiplies, fused multiply-adds and sums in the kept order)
+// and, with four blocks in flight, the two factorisations between and behind
+// the passes.  256 threads per block took, against this: 135 blocks 11.7 -> 8.3
+// us, 984 (1280x720) 37 -> 23.7, 2135 (1920x1080) 72 -> 44, 8349 (3840x2160)
+// 252 -> 175 us.
+template <int S, int G>
+struct FitterCqr2Shared {
+    uint4 tile[G][kTileChunks];   // 1024-byte aligned, for the swizzled copy
+    Cqr2Smem<S> sm[G];
+    alignas(16) float noise[kNoiseTableFloats];
+};
+
+template <int S, int G>
+__global__ void __launch_bounds__(kTeam * S * G, 1)
+    k_fitter_cqr2(int nblocks, int frame, NoiseConst nc, const __grid_constant__ CUtensorMap tmap,
+                  float* __restrict__ weights, float* __restrict__ mins_maxs, int* __restrict__ status) {
+    using Shared = FitterCqr2Shared<S, G>;
+    extern __shared__ unsigned char smem_raw[];
+    Shared& sh = *reinterpret_cast<Shared*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    constexpr uint32_t kTileBytes = kBuffers * kBlockPixels * sizeof(__half);
+    constexpr int kThreads = kTeam * S;
+    const int group = threadIdx.x / kThreads, bar = 1 + group, t = threadIdx.x % kThreads;
+    const bool leader = t == kThreads - 32;   // not in the warp that solves
+    const int first = group * gridDim.x + blockIdx.x, stride = G * gridDim.x;
+    Cqr2Smem<S>& sm = sh.sm[group];
+    uint4* tile = sh.tile[group];
+    auto issue = [&](int blk) {
+        fence_proxy_async();   // the tile was last read by generic loads
+        mbar_arrive_expect_tx(&sm.bar, kTileBytes);
+        tensor_copy_2d_g2s(tile, &tmap, 0, blk * kTileRows, &sm.bar);
+    };
+    if (leader) {
+        mbar_init(&sm.bar, 1);
+        fence_barrier_init();
+        sm.status = 0;
+    }
+    for (int e = threadIdx.x; e < kNoiseTableFloats; e += kThreads * G) sh.noise[e] = noise_quad_value(e, frame);
+    __syncthreads();
+    await_previous_kernel();
+    if (leader && first < nblocks) issue(first);
+
+    uint32_t phase = 0;
+    for (int b = first; b < nblocks; b += stride, phase ^= 1u) {
+        if (leader && !mbar_wait_bounded(&sm.bar, phase)) sm.status = kDevTimeout;
+        group_sync<S>(bar);
+        if (sm.status) {
+            if (leader) {
+                atomicExch(status, kDevTimeout);
+                mbar_wait_bounded(&sm.bar, phase);   // let the copy in flight land
+            }
+            return;
+        }
+        fit_cqr2<S>(reinterpret_cast<const unsigned char*>(tile), reinterpret_cast<const float4*>(sh.noise), nc.hi, t,
+                    sm, bar, weights + (size_t)b * kFeatures * 3, mins_maxs + (size_t)b * kScaled * 2, [&] {
+                        if (leader && b + stride < nblocks) issue(b + stride);
+                    });
+    }
+}
+
 // The frame's noise table in global memory (kNoiseTableFloats floats).
 __global__ void __launch_bounds__(256) k_noise_table(int frame, float* __restrict__ table) {
     await_previous_kernel();
@@ -324,20 +388,63 @@ static cudaError_t launch_rows16_t(int nblocks, int frame, NoiseConst nc, const 
                           map, weights, mins_maxs, status);
 }
 
+template <int S, int G>
+static cudaError_t launch_cqr2_t(int nblocks, int frame, NoiseConst nc, const CUtensorMap& map, float* weights,
+                                 float* mins_maxs, int* status, int dev, int sms, cudaStream_t s) {
+    auto kern = k_fitter_cqr2<S, G>;
+    const int smem = (int)sizeof(FitterCqr2Shared<S, G>) + 1024;   // + alignment slack
+    static std::atomic<bool> allowed[64];
+    if (!allowed[dev].load(std::memory_order_relaxed)) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        allowed[dev].store(true, std::memory_order_relaxed);
+    }
+    return launch_chained(kern, dim3(nblocks < sms ? nblocks : sms), dim3(kTeam * S * G), smem, s, nblocks, frame, nc,
+                          map, weights, mins_maxs, status);
+}
+
+// The current device and its SM count, looked up once per device.
+static cudaError_t device_sms(int* dev, int* sms) {
+    static std::atomic<int> sm_count[64];
+    cudaError_t e = cudaGetDevice(dev);
+    if (e != cudaSuccess) return e;
+    if (*dev < 0 || *dev >= 64) return cudaErrorInvalidDevice;
+    *sms = sm_count[*dev].load(std::memory_order_relaxed);
+    if (*sms == 0) {
+        e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, *dev);
+        if (e != cudaSuccess) return e;
+        sm_count[*dev].store(*sms, std::memory_order_relaxed);
+    }
+    return cudaSuccess;
+}
+
+static cudaError_t launch_cqr2(int nblocks, int frame, NoiseConst nc, const void* tmp, float* weights,
+                               float* mins_maxs, int* status, cudaStream_t s) {
+    if (nblocks <= 0) return cudaSuccess;
+    int dev = 0, sms = 0;
+    cudaError_t e = device_sms(&dev, &sms);
+    if (e != cudaSuccess) return e;
+    CUtensorMap map;
+    e = encode_tmp_map(tmp, nblocks, &map);
+    if (e != cudaSuccess) return e;
+    // Which shape for how many blocks per SM, as for k_fitter_rows16: up to
+    // three, several teams shorten a block's chain (144 blocks 8.4 us with four
+    // teams, 9.8 with two, 12.0 with one; 400 blocks 13.5 with two, 13.9 with
+    // one); beyond, one team per block leaves the fewest sums over threads
+    // (1050 blocks 23.8 us against 29.4 with two teams, 3680 blocks 79.6
+    // against 87.7).  Four groups of one team fill the registers (255 each).
+    const int per_sm = (nblocks + sms - 1) / sms;
+    if (per_sm <= 1) return launch_cqr2_t<4, 1>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
+    if (per_sm <= 3) return launch_cqr2_t<2, 3>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
+    return launch_cqr2_t<1, 4>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
+}
+
 static cudaError_t launch_rows16(int nblocks, int frame, NoiseConst nc, const void* tmp, float* weights,
                                  float* mins_maxs, int* status, cudaStream_t s) {
     if (nblocks <= 0) return cudaSuccess;
-    static std::atomic<int> sm_count[64];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    int dev = 0, sms = 0;
+    cudaError_t e = device_sms(&dev, &sms);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    int sms = sm_count[dev].load(std::memory_order_relaxed);
-    if (sms == 0) {
-        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return e;
-        sm_count[dev].store(sms, std::memory_order_relaxed);
-    }
     CUtensorMap map;
     e = encode_tmp_map(tmp, nblocks, &map);
     if (e != cudaSuccess) return e;
@@ -357,7 +464,7 @@ static cudaError_t launch_rows16(int nblocks, int frame, NoiseConst nc, const vo
     return launch_rows16_t<1, 6>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
 }
 
-bool fitter_reads_noise_table(bool half_tmp, int qr) { return !(half_tmp && qr == kFitReference); }
+bool fitter_reads_noise_table(bool half_tmp, int qr) { return !half_tmp || qr == kFitHouseholder32; }
 
 cudaError_t launch_fitter(const Geometry& g, int frame, NoiseConst nc, const void* tmp, bool half_tmp,
                           int qr, float* weights, float* mins_maxs, const float* noise_table, int* status,
@@ -366,21 +473,17 @@ cudaError_t launch_fitter(const Geometry& g, int frame, NoiseConst nc, const voi
     // The precision-form methods apply to binary16 tmp_data; float tmp_data
     // always takes the reference's arithmetic.
     if (half_tmp && qr == kFitReference) return launch_rows16(n, frame, nc, tmp, weights, mins_maxs, status, s);
+    if (half_tmp && qr == kFitCholQR2) return launch_cqr2(n, frame, nc, tmp, weights, mins_maxs, status, s);
     if (noise_table) {
         if (!half_tmp)
             return launch_fitter_t<false, kFitReference, true>(n, frame, nc, tmp, weights, mins_maxs, noise_table,
                                                                status, s);
-        if (qr == kFitCholQR2)
-            return launch_fitter_t<true, kFitCholQR2, true>(n, frame, nc, tmp, weights, mins_maxs, noise_table,
-                                                            status, s);
         return launch_fitter_t<true, kFitHouseholder32, true>(n, frame, nc, tmp, weights, mins_maxs, noise_table,
                                                               status, s);
     }
     if (!half_tmp)
         return launch_fitter_t<false, kFitReference, false>(n, frame, nc, tmp, weights, mins_maxs, nullptr, status,
                                                             s);
-    if (qr == kFitCholQR2)
-        return launch_fitter_t<true, kFitCholQR2, false>(n, frame, nc, tmp, weights, mins_maxs, nullptr, status, s);
     return launch_fitter_t<true, kFitHouseholder32, false>(n, frame, nc, tmp, weights, mins_maxs, nullptr, status,
                                                            s);
 }

@@ -43,8 +43,8 @@ cudaError_t launch_fitter_fp64(const Geometry& g, int frame, double noise_amount
 
 // status: device word that receives a nonzero code if a bounded wait ran out.
 // noise_table: the frame's table from launch_noise_table, or null to have
-// every CTA form it in shared memory (the reference's arithmetic on binary16
-// tmp_data always does: fitter_reads_noise_table).  qr: bmfr_params.fp32_qr (0 the
+// every CTA form it in shared memory (which the reference's arithmetic and
+// CholeskyQR2 on binary16 tmp_data always do: fitter_reads_noise_table).  qr: bmfr_params.fp32_qr (0 the
 // reference's arithmetic, 1 CholeskyQR2, 2 Householder in FP32).
 cudaError_t launch_fitter(const Geometry& g, int frame, NoiseConst nc, const void* tmp, bool half_tmp,
                           int qr, float* weights, float* mins_maxs, const float* noise_table, int* status,

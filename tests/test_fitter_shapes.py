@@ -1,4 +1,4 @@
-"""The reference-arithmetic fitter at every launch shape it takes.
+"""The reference-arithmetic and CholeskyQR2 fitters at every launch shape they take.
 
 The number of 32x32 blocks per SM decides how many teams share a block and
 how many blocks share an SM, so the sizes here lie on both sides of each
@@ -16,7 +16,7 @@ from oracle.oracle import Oracle
 pytestmark = pytest.mark.gpu
 
 
-def _draw(rng, blocks):
+def _draw(rng, blocks, special=True):
     t = np.empty((blocks, 13, 1024), np.float32)
     t[:, 0] = 1.0
     n = rng.standard_normal((blocks, 3, 1024))
@@ -25,7 +25,7 @@ def _draw(rng, blocks):
     t[:, 4:7] = rng.uniform(-4, 4, (blocks, 3, 1)) + scale * rng.standard_normal((blocks, 3, 1024))
     t[:, 7:10] = t[:, 4:7] ** 2
     t[:, 10:13] = rng.lognormal(-1.0, 1.5, (blocks, 3, 1024))
-    kind = rng.integers(0, 12, blocks)
+    kind = rng.integers(0, 12 if special else 2, blocks)
     t[kind == 0, 5] = 0.0                     # a plane: no range
     t[kind == 0, 8] = 0.0
     t[kind == 1, 10:13] = 0.0                 # black
@@ -36,6 +36,32 @@ def _draw(rng, blocks):
     t[kind == 5, 12, 17] = np.inf
     t[kind == 6, 6, 1000] = -np.inf
     return t
+
+
+# The precision form's stated errors against the FP64 fit: mean 1e-4, at most 2e-2.
+@pytest.mark.parametrize("W,H", [
+    (64, 48),       # 9 blocks: one per SM
+    (384, 320),     # 143
+    (416, 352),     # 168: up to three per SM
+    (672, 608),     # 440
+    (704, 640),     # 483: four groups per SM
+    (1600, 1024),   # 1683: three blocks each
+])
+def test_cholesky_qr2_shapes_match_fp64(cuda, W, H):
+    import torch
+    plan = B.Plan(W, H, fp32_qr=B.QR_CHOLESKY2)
+    blocks = plan.sizes.blocks
+    tmp = _draw(np.random.default_rng(W * 5 + H), blocks, special=False)
+    dev = torch.from_numpy(tmp.reshape(-1)).to(cuda)
+    w, mm, mm64 = (torch.empty(blocks, n, device=cuda) for n in (30, 12, 12))
+    w64 = torch.empty(blocks, 30, device=cuda, dtype=torch.float64)
+    B.fitter(plan, w, mm, dev, 5)
+    B.fitter_fp64(plan, w64, mm64, dev, 5)
+    assert torch.equal(mm, mm64)
+    err = (w.double() - w64).norm(dim=1) / w64.norm(dim=1).clamp(min=1e-3)
+    assert err.mean() < 1e-4 and err.max() < 2e-2, (err.mean().item(), err.max().item())
+    plan.check_device()
+    plan.close()
 
 
 @pytest.mark.parametrize("W,H,noise", [
