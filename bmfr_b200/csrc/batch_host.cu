@@ -295,6 +295,8 @@ cudaError_t launch_staged_step(bmfr_batch* b, const bmfr::BatchStepDesc& d, cuda
     std::sort(order.begin(), order.end(), [&](int x, int y) {
         return d.s[x].job.g.blocks > d.s[y].job.g.blocks;
     });
+    int blocks = 0;
+    for (int i = 0; i < d.n_streams; ++i) blocks += d.s[i].job.g.blocks;
     long long load[kStepWorkers] = {};
     bool used[kStepWorkers] = {};
     cudaError_t e = cudaEventRecord(b->fork, s);
@@ -321,7 +323,7 @@ cudaError_t launch_staged_step(bmfr_batch* b, const bmfr::BatchStepDesc& d, cuda
                                               fb.prev_spp, fb.cur_spp, J.tmp, ws);
         if (e == cudaSuccess)
             e = bmfr::launch_fitter(g, f, J.job.nc, J.tmp, half_tmp, b->p.fp32_qr, fb.weights, fb.mins_maxs,
-                                    fb.noise, b->d_status, ws);
+                                    fb.noise, b->d_status, ws, blocks - g.blocks);
         if (e == cudaSuccess)
             e = bmfr::launch_weighted_sum_accumulate(g, f, J.job.second_alpha, fb.weights, fb.mins_maxs, fb.cur_n,
                                                      fb.cur_p, nullptr, fb.prev_pix, fb.accept, fb.albedo,

@@ -79,10 +79,10 @@ struct bmfr_plan {
     bool uploaded[3] = {}, downloaded[2] = {}, done_recorded[3] = {};
     // bmfr_denoise_frames: the streams that run the accumulations of
     // overlapped frames (lowest priority) and the rest of each frame
-    // (highest priority), the end of frame f's accumulation (index f & 1),
-    // and the call's entry and exit on the caller's stream.
+    // (highest priority), the end of frame f's accumulation (index f & 1), of
+    // the last frame's fit, and the call's entry and exit on the caller's stream.
     cudaStream_t acc_stream = nullptr, frame_stream = nullptr;
-    cudaEvent_t ev_accumulated[2] = {}, ev_entry = nullptr, ev_exit = nullptr;
+    cudaEvent_t ev_accumulated[2] = {}, ev_fitted = nullptr, ev_entry = nullptr, ev_exit = nullptr;
     std::vector<void*> allocations;
 };
 
@@ -132,6 +132,7 @@ void free_plan(bmfr_plan* plan) {
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t& e : plan->ev_accumulated)
         if (e) cudaEventDestroy(e);
+    if (plan->ev_fitted) cudaEventDestroy(plan->ev_fitted);
     if (plan->ev_entry) cudaEventDestroy(plan->ev_entry);
     if (plan->ev_exit) cudaEventDestroy(plan->ev_exit);
     if (plan->acc_stream) cudaStreamDestroy(plan->acc_stream);
@@ -564,6 +565,7 @@ int run_frame(bmfr_plan* plan, const float* albedo, const float* cur_n, const fl
             e = bmfr::launch_fitter(g, f, bmfr::make_noise_const(plan->p.noise_amount), fs.tmp, half_tmp,
                                     plan->p.fp32_qr, plan->weights, plan->mins_maxs, fs.noise_table,
                                     plan->dev_status, s);
+        if (e == cudaSuccess && split) e = cudaEventRecord(plan->ev_fitted, s);
         mark(2);
     }
     // weighted_sum and accumulate_filtered_data in one pass per pixel; the
@@ -623,6 +625,7 @@ int ensure_overlap_resources(bmfr_plan* plan, cudaStream_t s) {
         e = cudaStreamCreateWithPriority(&plan->frame_stream, cudaStreamNonBlocking, greatest);
     for (int i = 0; i < 2 && e == cudaSuccess; ++i)
         if (!plan->ev_accumulated[i]) e = cudaEventCreateWithFlags(&plan->ev_accumulated[i], cudaEventDisableTiming);
+    if (e == cudaSuccess && !plan->ev_fitted) e = cudaEventCreateWithFlags(&plan->ev_fitted, cudaEventDisableTiming);
     if (e == cudaSuccess && !plan->ev_entry) e = cudaEventCreateWithFlags(&plan->ev_entry, cudaEventDisableTiming);
     if (e == cudaSuccess && !plan->ev_exit) e = cudaEventCreateWithFlags(&plan->ev_exit, cudaEventDisableTiming);
     if (e != cudaSuccess) return cuda_fail(e, "overlapped frames: stream and events");
@@ -675,6 +678,7 @@ int bmfr_denoise_frames(bmfr_plan* plan, int count, const bmfr_frame_io* io, con
     }
     cudaStream_t caller = (cudaStream_t)stream, s = caller;
     const bool overlap = count > 1 && plan->p.pipeline == BMFR_PIPELINE_STAGED && !plan->profiling;
+    const bool fit_first = bmfr::fitter_fills_gpu(plan->p.use_half_precision_in_tmp_data != 0, plan->p.fp32_qr);
     cudaStream_t sa = nullptr;
     if (overlap) {
         if (int st = ensure_overlap_resources(plan, caller)) return st;
@@ -702,6 +706,17 @@ int bmfr_denoise_frames(bmfr_plan* plan, int count, const bmfr_frame_io* io, con
         // set, and its accumulation precedes this one on the same stream.
         if (overlap && i >= 2) {
             cudaError_t e = cudaStreamWaitEvent(sa, plan->ev_frame_done[(f - 2) % 3], 0);
+            if (e != cudaSuccess) {
+                join_on_error();
+                return cuda_fail(e, "denoise_frames: frame order");
+            }
+        }
+        // A fitter that keeps every SM busy leaves the accumulation nothing to
+        // run on but SMs that the fitter then starts late on, so there the
+        // accumulation waits for frame f-1's fit and overlaps the stages
+        // behind it.
+        if (overlap && i >= 1 && fit_first) {
+            cudaError_t e = cudaStreamWaitEvent(sa, plan->ev_fitted, 0);
             if (e != cudaSuccess) {
                 join_on_error();
                 return cuda_fail(e, "denoise_frames: frame order");

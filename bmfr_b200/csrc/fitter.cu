@@ -375,7 +375,7 @@ static cudaError_t launch_fitter_t(int nblocks, int frame, NoiseConst nc, const 
 
 template <int S, int G>
 static cudaError_t launch_rows16_t(int nblocks, int frame, NoiseConst nc, const CUtensorMap& map, float* weights,
-                                   float* mins_maxs, int* status, int dev, int sms, cudaStream_t s) {
+                                   float* mins_maxs, int* status, int dev, int ctas, cudaStream_t s) {
     auto kern = k_fitter_rows16<S, G>;
     const int smem = (int)sizeof(FitterRows16Shared<G>) + 1024;   // + alignment slack
     static std::atomic<bool> allowed[64];
@@ -384,13 +384,13 @@ static cudaError_t launch_rows16_t(int nblocks, int frame, NoiseConst nc, const 
         if (e != cudaSuccess) return e;
         allowed[dev].store(true, std::memory_order_relaxed);
     }
-    return launch_chained(kern, dim3(nblocks < sms ? nblocks : sms), dim3(kTeam * S * G), smem, s, nblocks, frame, nc,
-                          map, weights, mins_maxs, status);
+    return launch_chained(kern, dim3(ctas), dim3(kTeam * S * G), smem, s, nblocks, frame, nc, map, weights, mins_maxs,
+                          status);
 }
 
 template <int S, int G>
 static cudaError_t launch_cqr2_t(int nblocks, int frame, NoiseConst nc, const CUtensorMap& map, float* weights,
-                                 float* mins_maxs, int* status, int dev, int sms, cudaStream_t s) {
+                                 float* mins_maxs, int* status, int dev, int ctas, cudaStream_t s) {
     auto kern = k_fitter_cqr2<S, G>;
     const int smem = (int)sizeof(FitterCqr2Shared<S, G>) + 1024;   // + alignment slack
     static std::atomic<bool> allowed[64];
@@ -399,8 +399,8 @@ static cudaError_t launch_cqr2_t(int nblocks, int frame, NoiseConst nc, const CU
         if (e != cudaSuccess) return e;
         allowed[dev].store(true, std::memory_order_relaxed);
     }
-    return launch_chained(kern, dim3(nblocks < sms ? nblocks : sms), dim3(kTeam * S * G), smem, s, nblocks, frame, nc,
-                          map, weights, mins_maxs, status);
+    return launch_chained(kern, dim3(ctas), dim3(kTeam * S * G), smem, s, nblocks, frame, nc, map, weights, mins_maxs,
+                          status);
 }
 
 // The current device and its SM count, looked up once per device.
@@ -418,8 +418,22 @@ static cudaError_t device_sms(int* dev, int* sms) {
     return cudaSuccess;
 }
 
+// Whether this launch and `beside` blocks of other streams fill the GPU: then
+// its blocks are packed onto as few SMs as they fill, with one team each,
+// instead of spread for the shortest time, because the SMs it leaves run the
+// others.  A step of eight 640x360 streams took 349 us spread and 294 packed
+// with CholeskyQR2, 503 and 370 with the reference's arithmetic; five streams
+// of 380 blocks together 184 spread and 193 packed.
+static bool fills_with_others(int nblocks, int beside, int sms) { return beside > 0 && nblocks + beside > 4 * sms; }
+
+// CTAs of `groups` groups that `nblocks` blocks fill, at most one per SM.
+static int packed_ctas(int nblocks, int groups, int sms) {
+    const int n = (nblocks + groups - 1) / groups;
+    return n < sms ? n : sms;
+}
+
 static cudaError_t launch_cqr2(int nblocks, int frame, NoiseConst nc, const void* tmp, float* weights,
-                               float* mins_maxs, int* status, cudaStream_t s) {
+                               float* mins_maxs, int* status, cudaStream_t s, int beside) {
     if (nblocks <= 0) return cudaSuccess;
     int dev = 0, sms = 0;
     cudaError_t e = device_sms(&dev, &sms);
@@ -433,14 +447,17 @@ static cudaError_t launch_cqr2(int nblocks, int frame, NoiseConst nc, const void
     // one); beyond, one team per block leaves the fewest sums over threads
     // (1050 blocks 23.8 us against 29.4 with two teams, 3680 blocks 79.6
     // against 87.7).  Four groups of one team fill the registers (255 each).
-    const int per_sm = (nblocks + sms - 1) / sms;
-    if (per_sm <= 1) return launch_cqr2_t<4, 1>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
-    if (per_sm <= 3) return launch_cqr2_t<2, 3>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
-    return launch_cqr2_t<1, 4>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
+    const int per_sm = (nblocks + sms - 1) / sms, spread = nblocks < sms ? nblocks : sms;
+    if (fills_with_others(nblocks, beside, sms))
+        return launch_cqr2_t<1, 4>(nblocks, frame, nc, map, weights, mins_maxs, status, dev,
+                                   packed_ctas(nblocks, 4, sms), s);
+    if (per_sm <= 1) return launch_cqr2_t<4, 1>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
+    if (per_sm <= 3) return launch_cqr2_t<2, 3>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
+    return launch_cqr2_t<1, 4>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
 }
 
 static cudaError_t launch_rows16(int nblocks, int frame, NoiseConst nc, const void* tmp, float* weights,
-                                 float* mins_maxs, int* status, cudaStream_t s) {
+                                 float* mins_maxs, int* status, cudaStream_t s, int beside) {
     if (nblocks <= 0) return cudaSuccess;
     int dev = 0, sms = 0;
     cudaError_t e = device_sms(&dev, &sms);
@@ -457,23 +474,28 @@ static cudaError_t launch_rows16(int nblocks, int frame, NoiseConst nc, const vo
     // 157.4 us with seven, 156.8 with six; 2200: 109.1 against 97.2), so there
     // are seven only where they take all blocks at once (986: 47.0 against
     // 57.8 us).
-    const int per_sm = (nblocks + sms - 1) / sms;
-    if (per_sm <= 1) return launch_rows16_t<4, 1>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
-    if (per_sm <= 3) return launch_rows16_t<2, 3>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
-    if (per_sm == 7) return launch_rows16_t<1, 7>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
-    return launch_rows16_t<1, 6>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, sms, s);
+    const int per_sm = (nblocks + sms - 1) / sms, spread = nblocks < sms ? nblocks : sms;
+    if (fills_with_others(nblocks, beside, sms))
+        return launch_rows16_t<1, 6>(nblocks, frame, nc, map, weights, mins_maxs, status, dev,
+                                     packed_ctas(nblocks, 6, sms), s);
+    if (per_sm <= 1) return launch_rows16_t<4, 1>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
+    if (per_sm <= 3) return launch_rows16_t<2, 3>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
+    if (per_sm == 7) return launch_rows16_t<1, 7>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
+    return launch_rows16_t<1, 6>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
 }
+
+bool fitter_fills_gpu(bool half_tmp, int qr) { return half_tmp && qr == kFitReference; }
 
 bool fitter_reads_noise_table(bool half_tmp, int qr) { return !half_tmp || qr == kFitHouseholder32; }
 
 cudaError_t launch_fitter(const Geometry& g, int frame, NoiseConst nc, const void* tmp, bool half_tmp,
                           int qr, float* weights, float* mins_maxs, const float* noise_table, int* status,
-                          cudaStream_t s) {
+                          cudaStream_t s, int beside) {
     const int n = g.blocks;
     // The precision-form methods apply to binary16 tmp_data; float tmp_data
     // always takes the reference's arithmetic.
-    if (half_tmp && qr == kFitReference) return launch_rows16(n, frame, nc, tmp, weights, mins_maxs, status, s);
-    if (half_tmp && qr == kFitCholQR2) return launch_cqr2(n, frame, nc, tmp, weights, mins_maxs, status, s);
+    if (half_tmp && qr == kFitReference) return launch_rows16(n, frame, nc, tmp, weights, mins_maxs, status, s, beside);
+    if (half_tmp && qr == kFitCholQR2) return launch_cqr2(n, frame, nc, tmp, weights, mins_maxs, status, s, beside);
     if (noise_table) {
         if (!half_tmp)
             return launch_fitter_t<false, kFitReference, true>(n, frame, nc, tmp, weights, mins_maxs, noise_table,

@@ -48,8 +48,14 @@ cudaError_t launch_fitter_fp64(const Geometry& g, int frame, double noise_amount
 // reference's arithmetic, 1 CholeskyQR2, 2 Householder in FP32).
 cudaError_t launch_fitter(const Geometry& g, int frame, NoiseConst nc, const void* tmp, bool half_tmp,
                           int qr, float* weights, float* mins_maxs, const float* noise_table, int* status,
-                          cudaStream_t s);
+                          cudaStream_t s, int beside = 0);
 cudaError_t launch_noise_table(int frame, float* table, cudaStream_t s);
+// Whether work beside launch_fitter's kernel only delays it: measured with the
+// next frame's accumulation beside it, us per frame against none: reference
+// arithmetic on binary16 tmp_data 1920x1080 203.7 / 197.9, 3840x2160 735.6 /
+// 692.7; CholeskyQR2 149.2 / 156.2, 547 / 565; float tmp_data 1280x720 126.1 /
+// 136.1.
+bool fitter_fills_gpu(bool half_tmp, int qr);
 // Whether launch_fitter reads `noise_table`, so that a frame has to make it.
 bool fitter_reads_noise_table(bool half_tmp, int qr);
 // One CTA waits, with the fitter's bounded wait limited to limit_ns, on a
