@@ -14,14 +14,12 @@
 // so that the first stage of the reference's reduction tree (ids i, i+64,
 // i+128, i+192, bmfr.cl:32-33) sits inside one warp and runs on shuffles.
 //
-// Reductions.  block_reduce (min/max), block_sum_dots and block_sum1_all
-// evaluate parallel_reduction_sum/min/max (bmfr.cl:25-87) over exactly the
-// same tree, so the sums round exactly as the reference's do.  The batched
-// forms reduce up to 12 independent values behind one pair of barriers: the
-// twelve min/max values of the scaling step, and per column the up to twelve
-// dot products, which are independent once the Householder vector is known.
-// A column costs the norm (one barrier) and the dots (two) where the
-// reference spends three barriers per dot product.
+// Reductions.  block_sum_dots and block_sum1_all evaluate
+// parallel_reduction_sum (bmfr.cl:25-43) over exactly the same tree, so the
+// sums round exactly as the reference's do.  A column's up to twelve dot
+// products, which are independent once the Householder vector is known, share
+// one pair of barriers: a column costs the norm (one barrier) and the dots
+// (two) where the reference spends three barriers per dot product.
 //
 // Columns run in a loop; each column's update writes later column k into
 // tile slot k - 1, so the tile moves down by one column as it is updated and
@@ -77,61 +75,6 @@ __device__ __forceinline__ int work_item_id() {
     return 8 * warp + (lane & 7) + 64 * (lane >> 3);
 }
 
-template <int OP>
-__device__ __forceinline__ float rop(float a, float b) {
-    if (OP == 0) return a + b;
-    if (OP == 1) return fmin_cl(a, b);
-    return fmax_cl(a, b);
-}
-
-// Batched work-group min/max reduction of n <= VMAX values per thread
-// (parallel_reduction_min/max, bmfr.cl:45-87).  Values [0, split) use OP_A,
-// [split, n) use OP_B (1 min, 2 max); results in sm.out.
-template <int VMAX, int OP_A, int OP_B>
-__device__ __forceinline__ void block_reduce(const float (&v)[VMAX], int n, int split, FitterSmem& sm) {
-    static_assert(OP_A != 0 && OP_B != 0, "sums go through block_sum_dots or block_sum1_all");
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-    for (int i = 0; i < VMAX; ++i) {
-        if (i < n) {
-            const float a = v[i];
-            const float b = __shfl_down_sync(kFull, a, 8);
-            const float c = __shfl_down_sync(kFull, a, 16);
-            const float d = __shfl_down_sync(kFull, a, 24);
-            const int op = i < split ? OP_A : OP_B;
-            float s1;
-            if (op == 1) s1 = fmin_cl(fmin_cl(fmin_cl(a, b), c), d);    // bmfr.cl:52-53
-            else s1 = fmax_cl(fmax_cl(fmax_cl(a, b), c), d);            // bmfr.cl:74-75
-            if (lane < 8) sm.part[i * kPartStride + 8 * warp + lane] = s1;
-        }
-    }
-    __syncthreads();
-    // Stages 2 and 3: value vi is finished by the 8-lane group `lane >> 3` of
-    // warp vi % 8; lane j of the group forms the j-th second-stage value
-    // (bmfr.cl:56-58), lane 0 of the group the result (bmfr.cl:60-63).
-    const int vi = warp + 8 * (lane >> 3);
-    const int j = lane & 7;
-    const int op = vi < split ? OP_A : OP_B;
-    float s2 = 0.0f;
-    if (vi < n) {
-        const float* p = sm.part + vi * kPartStride + j;
-        float acc = p[0];
-#pragma unroll
-        for (int m = 1; m < 8; ++m) acc = op == 1 ? fmin_cl(acc, p[8 * m]) : fmax_cl(acc, p[8 * m]);
-        s2 = acc;
-    }
-    if (warp < n) {   // warp-uniform: warps without a value skip
-        float r = __shfl_sync(kFull, s2, 0, 8);
-#pragma unroll
-        for (int m = 1; m < 8; ++m) {
-            const float x = __shfl_sync(kFull, s2, m, 8);
-            r = op == 1 ? fmin_cl(r, x) : fmax_cl(r, x);
-        }
-        if (vi < n && j == 0) sm.out[vi] = r;
-    }
-    __syncthreads();
-}
-
 // parallel_reduction_sum (bmfr.cl:25-43) of the column step's n <= VMAX dot
 // products; results in sm.out.  NMIN is a compile-time lower bound on n: the
 // guards of the values below it vanish.  Returns, from the closing barrier,
@@ -143,7 +86,7 @@ __device__ __forceinline__ void block_reduce(const float (&v)[VMAX], int n, int 
 // of ids i and i+192 (groups 0 and 3) swap the other half and each receive
 // b + c from their neighbour group, so group 0 finishes values [0, H) and
 // group 3 values [H, 2H) as a + ((b + c) + d): one shuffle per value instead
-// of three.  Stages 2 and 3 as in block_reduce.
+// of three.
 template <int VMAX, int NMIN>
 __device__ __forceinline__ bool block_sum_dots(const float (&v)[VMAX], int n, FitterSmem& sm) {
     constexpr int H = (VMAX + 1) / 2;
@@ -343,17 +286,50 @@ __device__ __forceinline__ float2 add_noise_r2(float2 v, float2 r, NoiseConst c)
     return add2(sm, add2(se, pl));
 }
 
+// value + NOISE_AMOUNT*2*r rounded once, as add_noise_r2 gives it, for
+// binary16 values and |NOISE_AMOUNT| < 1.  Every binary16 value is then a
+// multiple of the last place of p = RN(hi*r), so s - v is exact (Dekker's fast
+// two-sum) and one fused multiply-add gives what s misses of v + hi*r.
+__device__ __forceinline__ float2 add_noise_half2(float2 v, float2 r, NoiseConst c) {
+    const float2 hi = dup2(c.hi);
+    const float2 s = add2(v, rmul2(hi, r, c.neg_zero));
+    const float2 left = fma2(hi, r, fma2(s, dup2(-1.0f), v));
+    return add2(s, fma2(dup2(c.lo), r, left));
+}
+
+// Quotients n / b of two numerators, negated: Markstein's correction as
+// described above (ny = -RN(1/b)); the sign of a zero quotient is kept.
+__device__ __forceinline__ float2 neg_quotient(float2 n, float2 ny, float2 b) {
+    const float2 nq = mul2(n, ny);
+    const float2 r = fma2(nq, b, n);
+    return fma2(r, ny, nq);
+}
+
+// Minimum or maximum over the warp; NaN operands are ignored, as fmin/fmax do.
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 // Column k of the tile as two float pairs (rows q0,q1 and q2,q3), with the
-// first column's noise added to features 1..9 (bmfr.cl:625-627).
-template <bool HALF, bool NOISE>
+// first column's noise added to features 1..9 (bmfr.cl:625-627).  PLAIN: the
+// noise is below 1.
+template <bool HALF, bool NOISE, bool PLAIN = false>
 __device__ __forceinline__ void load_column(const Tile<HALF>& t, int k, int fb, const float* __restrict__ noise,
                                             NoiseConst nc, float2& a01, float2& a23) {
     a01 = t.get2(k, 0);
     a23 = t.get2(k, 1);
     if (NOISE && fb < kFeatures) {
         const float* r = noise + (fb - 1) * 4 * kLocal + threadIdx.x;
-        a01 = add_noise_r2(a01, make_float2(r[0], r[kLocal]), nc);
-        a23 = add_noise_r2(a23, make_float2(r[2 * kLocal], r[3 * kLocal]), nc);
+        const float2 r01 = make_float2(r[0], r[kLocal]), r23 = make_float2(r[2 * kLocal], r[3 * kLocal]);
+        a01 = HALF && PLAIN ? add_noise_half2(a01, r01, nc) : add_noise_r2(a01, r01, nc);
+        a23 = HALF && PLAIN ? add_noise_half2(a23, r23, nc) : add_noise_r2(a23, r23, nc);
     }
 }
 
@@ -366,7 +342,10 @@ __device__ __forceinline__ void load_column(const Tile<HALF>& t, int k, int fb, 
 // VS: column slots the loops visit (a compile-time bound >= the V later
 // columns): the late columns take a shorter instance.  VMIN: a compile-time
 // bound <= V, so that the slots below it are visited without a guard.
-template <bool HALF, bool NOISE, int VS = 12, int VMIN = 0>
+// PLAIN (the first column): it is all ones, as in every frame the pipeline
+// makes, so one quotient per later column serves every row but row 0; and the
+// noise is below 1.
+template <bool HALF, bool NOISE, int VS = 12, int VMIN = 0, bool PLAIN = false>
 __device__ __forceinline__ void qr_column(Tile<HALF>& t, int col, int id, const float* __restrict__ noise,
                                           NoiseConst nc, FitterSmem& sm) {
     const int V = kBuffers - 1 - col;
@@ -434,8 +413,17 @@ __device__ __forceinline__ void qr_column(Tile<HALF>& t, int col, int id, const 
             d[i] = d[i + 1] = 0.0f;
             if (i < VMIN || i < V) {
                 float2 a01, a23, b01, b23;
-                load_column<HALF, NOISE>(t, i + 1, i + 1, noise, nc, a01, a23);
-                load_column<HALF, NOISE>(t, i + 2, i + 2, noise, nc, b01, b23);
+                load_column<HALF, NOISE, PLAIN>(t, i + 1, i + 1, noise, nc, a01, a23);
+                load_column<HALF, NOISE, PLAIN>(t, i + 2, i + 2, noise, nc, b01, b23);
+                if (PLAIN) {   // u is 1 but in row 0
+                    const float2 p0 = id == 0 ? rmul2(make_float2(a01.x, b01.x), dup2(u0), nc.neg_zero)
+                                              : make_float2(a01.x, b01.x);
+                    float2 s = add2(add2(dup2(0.0f), p0), make_float2(a01.y, b01.y));
+                    s = add2(add2(s, make_float2(a23.x, b23.x)), make_float2(a23.y, b23.y));
+                    d[i] = s.x;
+                    d[i + 1] = s.y;
+                    continue;
+                }
                 float2 s = add2(dup2(0.0f), rmul2(make_float2(a01.x, b01.x), uq0, nc.neg_zero));
                 s = add2(s, rmul2(make_float2(a01.y, b01.y), uq1, nc.neg_zero));
                 s = add2(s, rmul2(make_float2(a23.x, b23.x), uq2, nc.neg_zero));
@@ -479,10 +467,14 @@ __device__ __forceinline__ void qr_column(Tile<HALF>& t, int col, int id, const 
         for (int i = 0; i < VS; ++i) {
             if (i < VMIN || i < V) {
                 const float2 d2 = dup2(sm.out[i]);
-                const float2 num01 = mul2(u2_01, d2), num23 = mul2(u2_23, d2);
-                const float2 nq01 = mul2(num01, ny), nq23 = mul2(num23, ny);
-                const float2 r01 = fma2(nq01, b2, num01), r23 = fma2(nq23, b2, num23);
-                const float2 mq01 = fma2(r01, ny, nq01), mq23 = fma2(r23, ny, nq23);   // -RN(num / uls)
+                float2 mq01, mq23;   // -RN(num / uls)
+                if constexpr (PLAIN) {
+                    mq01 = neg_quotient(make_float2(u2_01.x * d2.x, u2_01.y * d2.y), ny, b2);
+                    mq23 = dup2(mq01.y);
+                } else {
+                    mq01 = neg_quotient(mul2(u2_01, d2), ny, b2);
+                    mq23 = neg_quotient(mul2(u2_23, d2), ny, b2);
+                }
                 if constexpr (HALF && !NOISE) {
                     // a - q straight from the binary16 a (add.f32.f16); row
                     // id keeps its half when it lies above the column.
@@ -494,7 +486,7 @@ __device__ __forceinline__ void qr_column(Tile<HALF>& t, int col, int id, const 
                                                       add_f32_h(__high2half(h23), mq23.y));
                 } else {
                     float2 a01, a23;
-                    load_column<HALF, NOISE>(t, i + 1, i + 1, noise, nc, a01, a23);
+                    load_column<HALF, NOISE, PLAIN>(t, i + 1, i + 1, noise, nc, a01, a23);
                     float2 n01 = add2(a01, mq01);
                     const float2 n23 = add2(a23, mq23);
                     if (!row0) n01.x = a01.x;
@@ -511,7 +503,7 @@ __device__ __forceinline__ void qr_column(Tile<HALF>& t, int col, int id, const 
                 const float ad = fabsf(dot);
                 const bool fast = fast_u && (ad == 0.0f || (ad >= 0x1p-32f && ad <= 0x1p30f));
                 float2 a01, a23;
-                load_column<HALF, NOISE>(t, i + 1, i + 1, noise, nc, a01, a23);
+                load_column<HALF, NOISE, PLAIN>(t, i + 1, i + 1, noise, nc, a01, a23);
                 float2 n01, n23;
                 if (fast) {
                     const float2 d2 = dup2(dot);
@@ -977,35 +969,65 @@ __device__ __forceinline__ void fit_block(Tile<HALF>& t, const float* __restrict
             fit_columns_fast(t, id, noise, nc, sm);
         }
     } else {
-        // Min/max scaling of features 4..9 (bmfr.cl:511-542), the
-        // reference's reduction tree.
-        float mm[12];
+        // Min/max of features 4..9 (bmfr.cl:511-535): over the warp in one
+        // operation, then lane v < 12 of every warp over the eight warps.
+        // Minima and maxima are exact in any order; only the sign of a zero
+        // bound can differ from the reference's tree.
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        bool ones = true;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float2 x = t.get2(0, h);
+            ones = ones && x.x == 1.0f && x.y == 1.0f;
+        }
 #pragma unroll
         for (int f = 0; f < kScaled; ++f) {
             const float2 a01 = t.get2(kNotScaled + f, 0), a23 = t.get2(kNotScaled + f, 1);
-            const float a[4] = {a01.x, a01.y, a23.x, a23.y};
-            float mx = -INFINITY, mn = INFINITY;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                mx = fmax_cl(a[q], mx);
-                mn = fmin_cl(a[q], mn);
+            const float hi = warp_max(fmaxf(-INFINITY, fmaxf(fmaxf(a01.x, a01.y), fmaxf(a23.x, a23.y))));
+            const float lo = warp_min(fminf(INFINITY, fminf(fminf(a01.x, a01.y), fminf(a23.x, a23.y))));
+            if (lane == 0) {
+                sm.part[12 * warp + f] = hi;
+                sm.part[12 * warp + kScaled + f] = lo;
             }
-            mm[f] = mx;
-            mm[kScaled + f] = mn;
         }
-        block_reduce<12, 2, 1>(mm, 12, kScaled, sm);
-        if (threadIdx.x < 2 * kScaled) {
-            const int f = threadIdx.x >> 1;
-            mm_out[threadIdx.x] = (threadIdx.x & 1) ? sm.out[f] : sm.out[kScaled + f];
+        ones = __syncthreads_and(ones) != 0;
+        const int mine = lane < 12 ? lane : 0;
+        float bound = sm.part[mine];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) {
+            const float x = sm.part[12 * w + mine];
+            bound = mine < kScaled ? fmaxf(bound, x) : fminf(bound, x);
         }
+        if (warp == 0 && lane < 12) mm_out[lane < kScaled ? 2 * lane + 1 : 2 * (lane - kScaled)] = bound;
+        // scale() (bmfr.cl:200-205), rounded at the store (bmfr.cl:540).  The
+        // bounds of binary16 values leave every numerator in the range of
+        // Markstein's correction unless the range is infinite, which divides
+        // finite numerators to zero and the others to NaN.
 #pragma unroll
         for (int f = 0; f < kScaled; ++f) {
-            const float bmax = sm.out[f], bmin = sm.out[kScaled + f];
+            const float bmax = __shfl_sync(kFull, bound, f), bmin = __shfl_sync(kFull, bound, kScaled + f);
             const float2 a01 = t.get2(kNotScaled + f, 0), a23 = t.get2(kNotScaled + f, 1);
-            t.set2(kNotScaled + f, 0, scale_by(a01.x, bmin, bmax), scale_by(a01.y, bmin, bmax));
-            t.set2(kNotScaled + f, 1, scale_by(a23.x, bmin, bmax), scale_by(a23.y, bmin, bmax));
+            if constexpr (HALF) {
+                const float d = bmax - bmin;
+                float2 n01 = add2(a01, dup2(-bmin)), n23 = add2(a23, dup2(-bmin));
+                if (fabsf(d) > 0x1p60f) {
+                    n01 = mul2(n01, dup2(0.0f));
+                    n23 = mul2(n23, dup2(0.0f));
+                } else if (fabsf(d) > 1.0f) {
+                    const float2 ny = dup2(-__frcp_rn(d));
+                    n01 = neg2(neg_quotient(n01, ny, dup2(d)));
+                    n23 = neg2(neg_quotient(n23, ny, dup2(d)));
+                }
+                t.set2(kNotScaled + f, 0, n01.x, n01.y);
+                t.set2(kNotScaled + f, 1, n23.x, n23.y);
+            } else {
+                t.set2(kNotScaled + f, 0, scale_by(a01.x, bmin, bmax), scale_by(a01.y, bmin, bmax));
+                t.set2(kNotScaled + f, 1, scale_by(a23.x, bmin, bmax), scale_by(a23.y, bmin, bmax));
+            }
         }
-        qr_column<HALF, true>(t, 0, id, noise, nc, sm);
+        __syncthreads();   // sm.part is read; the first column's sums go there
+        if (ones && fabsf(nc.hi) < 2.0f) qr_column<HALF, true, 12, 12, true>(t, 0, id, noise, nc, sm);
+        else qr_column<HALF, true, 12, 12>(t, 0, id, noise, nc, sm);
 #pragma unroll 1
         for (int col = 1; col < 6; ++col) qr_column<HALF, false, 12, 7>(t, col, id, noise, nc, sm);   // 11..7 later columns
 #pragma unroll 1

@@ -66,18 +66,6 @@ __device__ __forceinline__ float noise16_value(int entry, int frame) {
     return hash_random(noise_index(row, 0, fq / 4 + 1, frame)) - 0.5f;
 }
 
-// Minimum or maximum over the warp; NaN operands are ignored, as fmin/fmax do.
-__device__ __forceinline__ float warp_min(float v) {
-    float r;
-    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
-}
-__device__ __forceinline__ float warp_max(float v) {
-    float r;
-    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
-}
-
 // Stages 2 and 3 of parallel_reduction_sum (bmfr.cl:35-42) on the 64
 // first-stage sums at p: lane j of an 8-lane group forms sum_vec[j], then
 // every lane adds the eight left to right.
@@ -160,17 +148,6 @@ __device__ __forceinline__ float dot_rows(const Rows& x, const Rows& u, float u0
     return s0 + ((s1 + s2) + s3);   // bmfr.cl:33
 }
 
-// value + NOISE_AMOUNT*2*r rounded once, as add_noise_r2 gives it, for
-// binary16 values and |NOISE_AMOUNT| < 1.  Every binary16 value is then a
-// multiple of the last place of p = RN(hi*r), so s - v is exact (Dekker's fast
-// two-sum) and one fused multiply-add gives what s misses of v + hi*r.
-__device__ __forceinline__ float2 add_noise_half2(float2 v, float2 r, NoiseConst c) {
-    const float2 hi = dup2(c.hi);
-    const float2 s = add2(v, rmul2(hi, r, c.neg_zero));
-    const float2 left = fma2(hi, r, fma2(s, dup2(-1.0f), v));
-    return add2(s, fma2(dup2(c.lo), r, left));
-}
-
 // The column as float pairs with the first column's noise added to features
 // 1..9 (bmfr.cl:625-627).
 template <bool PLAIN>
@@ -186,14 +163,6 @@ __device__ __forceinline__ void noised_rows(const Rows& x, int k, int i, const f
         a[2 * q] = PLAIN ? add_noise_half2(a[2 * q], r01, nc) : add_noise_r2(a[2 * q], r01, nc);
         a[2 * q + 1] = PLAIN ? add_noise_half2(a[2 * q + 1], r23, nc) : add_noise_r2(a[2 * q + 1], r23, nc);
     }
-}
-
-// Quotients n / b of two numerators, negated: Markstein's correction as in
-// fit_block.cuh (ny = -RN(1/b)); the sign of a zero quotient is kept.
-__device__ __forceinline__ float2 neg_quotient(float2 n, float2 ny, float2 b) {
-    const float2 nq = mul2(n, ny);
-    const float2 r = fma2(nq, b, n);
-    return fma2(r, ny, nq);
 }
 
 // The Householder vector of a finished column and what its update divides by.

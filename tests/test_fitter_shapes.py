@@ -91,3 +91,35 @@ def test_fitter_shapes_match_oracle(cuda, W, H, noise):
     np.testing.assert_array_equal(w.cpu().numpy(), want_w)
     plan.check_device()
     plan.close()
+
+
+@pytest.mark.parametrize("noise", [1e-2, 1.5])
+def test_float_tmp_data_matches_oracle(cuda, noise):
+    """First columns that are and are not the constant feature, noise on both sides of 1."""
+    import torch
+    W, H = 320, 200
+    o = Oracle(W, H, use_half=False, noise_amount=noise)
+    plan = B.Plan(W, H, use_half_precision_in_tmp_data=0, noise_amount=noise)
+    tmp = np.nan_to_num(_draw(np.random.default_rng(3), o.blocks).astype(np.float32), posinf=1.0, neginf=-1.0)
+    want_w, want_mm = np.zeros(o.blocks * 30, np.float32), np.zeros(o.blocks * 12, np.float32)
+    o.fitter(want_w, want_mm, tmp.reshape(-1).copy(), 5)
+    w, mm = torch.empty(o.blocks * 30, device=cuda), torch.empty(o.blocks * 12, device=cuda)
+    B.fitter(plan, w, mm, torch.from_numpy(tmp.reshape(-1)).to(cuda), 5)
+    np.testing.assert_array_equal(mm.cpu().numpy(), want_mm)
+    np.testing.assert_array_equal(w.cpu().numpy(), want_w)
+    plan.close()
+
+
+def test_fused_pipeline_with_large_noise_matches_staged(cuda):
+    W, H = 96, 80
+    sc = B.Scene(5, W, H, 8)
+    got = []
+    for pipeline in (B.PIPELINE_STAGED, B.PIPELINE_FUSED):
+        plan = B.Plan(W, H, noise_amount=1.5, pipeline=pipeline)
+        for f in range(3):
+            d = sc.render(f)
+            plan.upload_frame(d["albedo"], d["normals"], d["positions"], d["noisy"])
+            plan.denoise_frame(sc.prev_camera(f), sc.pixel_offset(f))
+        got.append(plan.download_result())
+        plan.close()
+    np.testing.assert_array_equal(got[0], got[1])
