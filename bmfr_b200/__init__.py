@@ -57,21 +57,21 @@ def _stream_ptr(stream) -> C.c_void_p:
     return C.c_void_p(stream.cuda_stream)
 
 
-def _ptr(t, name: str, nbytes: int | None = None, optional: bool = False) -> C.c_void_p:
-    """Device pointer of a contiguous CUDA tensor (or None)."""
+def _ptr(t, name: str, nbytes: int | None = None, optional: bool = False) -> int | None:
+    """Device address of a contiguous CUDA tensor (or None)."""
     if t is None:
         if optional:
-            return C.c_void_p(None)
+            return None
         raise ValueError(f"{name} must not be None")
     if isinstance(t, int):
-        return C.c_void_p(t)
+        return t
     if not t.is_cuda:
         raise ValueError(f"{name} must be a CUDA tensor")
     if not t.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
-    if nbytes is not None and t.numel() * t.element_size() < nbytes:
-        raise ValueError(f"{name} holds {t.numel() * t.element_size()} bytes, needs {nbytes}")
-    return C.c_void_p(t.data_ptr())
+    if nbytes is not None and t.nbytes < nbytes:
+        raise ValueError(f"{name} holds {t.nbytes} bytes, needs {nbytes}")
+    return t.data_ptr()
 
 
 def _mem_ptr(t, name: str, nbytes: int | None = None) -> C.c_void_p:
@@ -91,10 +91,21 @@ def _mem_ptr(t, name: str, nbytes: int | None = None) -> C.c_void_p:
     return _ptr(t, name, nbytes)
 
 
+_FLOATS = {n: C.c_float * n for n in (2, 16)}
+
+
 def _f32(values, n: int, name: str):
-    a = np.ascontiguousarray(np.asarray(values, dtype=np.float32).reshape(-1))
+    """`values` as n float32 in host memory, and the pointer to pass.  The
+    small arrays of every call (a matrix, an offset) are viewed in place where
+    they can be: an ndarray's .ctypes costs more than the rest of the call's
+    conversions together."""
+    a = values
+    if type(a) is not np.ndarray or a.dtype != np.float32 or not a.flags.c_contiguous:
+        a = np.ascontiguousarray(np.asarray(values, dtype=np.float32).reshape(-1))
     if a.size != n:
         raise ValueError(f"{name} needs {n} floats")
+    if n in _FLOATS and a.flags.writeable:
+        return a, _FLOATS[n].from_buffer(a)
     return a, a.ctypes.data_as(C.POINTER(C.c_float))
 
 
