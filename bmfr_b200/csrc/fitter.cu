@@ -467,20 +467,24 @@ static cudaError_t launch_rows16(int nblocks, int frame, NoiseConst nc, const vo
     if (e != cudaSuccess) return e;
     // Which shape for how many blocks per SM.  Up to three, one block's chain of
     // ten columns is what takes the time, and several teams shorten it: 100
-    // blocks 17.3 us with four teams, 18.6 with two, 23.5 with one; 400 blocks
-    // 26.6 us with two, 29.8 with one.  Beyond, one team per block costs the
-    // fewest operations: 600 blocks 37.6 us against 44.2 with two teams.  A
-    // seventh group overloads two of the SM's four schedulers (3680 blocks:
-    // 157.4 us with seven, 156.8 with six; 2200: 109.1 against 97.2), so there
-    // are seven only where they take all blocks at once (986: 47.0 against
-    // 57.8 us).
+    // blocks 16.6 us with four teams, 17.5 with two, 21.7 with one; 400 blocks
+    // 24.7 us with two, 27.5 with one.  Beyond, one team per block costs the
+    // fewest operations: 600 blocks 33.9 us against 41.0 with two teams.  A
+    // seventh group overloads two of the SM's four schedulers, so a round of
+    // seven blocks lasts longer than one of six (3108 blocks: 38.6 against
+    // 29.3 us) and pays only where it saves a whole round: 986 blocks 42.3
+    // against 52.9 us, 1904 72.0 against 82.2, 2072 79.0 against 82.4, 2812
+    // 108.7 against 112.0, 3108 115.9 against 117.2; but 1776 72.0 against
+    // 64.1, 2100 96.8 against 86.8, and above 21 blocks per SM the saved round
+    // no longer makes up for the longer ones (4144: 153.6 against 147.9).
     const int per_sm = (nblocks + sms - 1) / sms, spread = nblocks < sms ? nblocks : sms;
     if (fills_with_others(nblocks, beside, sms))
         return launch_rows16_t<1, 6>(nblocks, frame, nc, map, weights, mins_maxs, status, dev,
                                      packed_ctas(nblocks, 6, sms), s);
     if (per_sm <= 1) return launch_rows16_t<4, 1>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
     if (per_sm <= 3) return launch_rows16_t<2, 3>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
-    if (per_sm == 7) return launch_rows16_t<1, 7>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
+    if (per_sm <= 21 && (per_sm + 6) / 7 < (per_sm + 5) / 6)
+        return launch_rows16_t<1, 7>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
     return launch_rows16_t<1, 6>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
 }
 

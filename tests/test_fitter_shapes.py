@@ -74,6 +74,7 @@ def test_cholesky_qr2_shapes_match_fp64(cuda, W, H):
     (1056, 960, 1e-2),    # 1054
     (1280, 720, 1e-2),    # 984: seven per SM
     (1600, 1024, 1e-2),   # 1683: two blocks per group
+    (1760, 1056, 1e-2),   # 1904: seven groups, two rounds
     (64, 48, 0.0),
     (64, 48, 1.5),        # noise beyond the fast two-sum
 ])
