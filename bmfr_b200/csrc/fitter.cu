@@ -216,7 +216,19 @@ __global__ void __launch_bounds__(kTeam * S * G, 1)
 // and, with four blocks in flight, the two factorisations between and behind
 // the passes.  256 threads per block took, against this: 135 blocks 11.7 -> 8.3
 // us, 984 (1280x720) 37 -> 23.7, 2135 (1920x1080) 72 -> 44, 8349 (3840x2160)
-// 252 -> 175 us.
+// 252 -> 152 us.
+//
+// The fit is straight-line code that each group passes once per block, and
+// waiting for instructions is its longest stall (1.3 cycles per issue).  Groups
+// that have drifted apart fetch it four times over, so from the seventh round
+// on it pays to bring them back together (ALIGNED: a barrier of the CTA every
+// fourth round): 3680 blocks 79.0 -> 75.2 us, 4736 101 -> 90.5, 8228 179 -> 153
+// (156 with a barrier at every round from the fifth on, 152.4 at every second
+// round).  In fewer rounds the groups still run side by side and the loop costs
+// more than it gives (3000 blocks, six rounds, 63.7 -> 64.1 us; 2400, five, 52.8
+// -> 53.5; 2135, four, 44.0 -> 45.2).
+constexpr int kAlignRounds = 4;
+
 template <int S, int G>
 struct FitterCqr2Shared {
     uint4 tile[G][kTileChunks];   // 1024-byte aligned, for the swizzled copy
@@ -224,7 +236,7 @@ struct FitterCqr2Shared {
     alignas(16) float noise[kNoiseTableFloats];
 };
 
-template <int S, int G>
+template <int S, int G, bool ALIGNED>
 __global__ void __launch_bounds__(kTeam * S * G, 1)
     k_fitter_cqr2(int nblocks, int frame, NoiseConst nc, const __grid_constant__ CUtensorMap tmap,
                   float* __restrict__ weights, float* __restrict__ mins_maxs, int* __restrict__ status) {
@@ -253,8 +265,7 @@ __global__ void __launch_bounds__(kTeam * S * G, 1)
     await_previous_kernel();
     if (leader && first < nblocks) issue(first);
 
-    uint32_t phase = 0;
-    for (int b = first; b < nblocks; b += stride, phase ^= 1u) {
+    auto fit = [&](int b, uint32_t phase) {   // false: the block's copy did not arrive
         if (leader && !mbar_wait_bounded(&sm.bar, phase)) sm.status = kDevTimeout;
         group_sync<S>(bar);
         if (sm.status) {
@@ -262,12 +273,27 @@ __global__ void __launch_bounds__(kTeam * S * G, 1)
                 atomicExch(status, kDevTimeout);
                 mbar_wait_bounded(&sm.bar, phase);   // let the copy in flight land
             }
-            return;
+            return false;
         }
         fit_cqr2<S>(reinterpret_cast<const unsigned char*>(tile), reinterpret_cast<const float4*>(sh.noise), nc.hi, t,
                     sm, bar, weights + (size_t)b * kFeatures * 3, mins_maxs + (size_t)b * kScaled * 2, [&] {
                         if (leader && b + stride < nblocks) issue(b + stride);
                     });
+        return true;
+    };
+    if constexpr (ALIGNED) {
+        // The number of rounds is the same in every thread of the CTA; a group
+        // without a block left, or whose copy failed, only joins the barriers.
+        const int rounds = (nblocks - (int)blockIdx.x + stride - 1) / stride;
+        bool live = true;
+        for (int r = 0, b = first; r < rounds; ++r, b += stride) {
+            if (r % kAlignRounds == kAlignRounds - 1) __syncthreads();
+            if (live && b < nblocks) live = fit(b, r & 1);
+        }
+    } else {
+        uint32_t phase = 0;
+        for (int b = first; b < nblocks; b += stride, phase ^= 1u)
+            if (!fit(b, phase)) return;
     }
 }
 
@@ -388,10 +414,10 @@ static cudaError_t launch_rows16_t(int nblocks, int frame, NoiseConst nc, const 
                           status);
 }
 
-template <int S, int G>
+template <int S, int G, bool ALIGNED = false>
 static cudaError_t launch_cqr2_t(int nblocks, int frame, NoiseConst nc, const CUtensorMap& map, float* weights,
                                  float* mins_maxs, int* status, int dev, int ctas, cudaStream_t s) {
-    auto kern = k_fitter_cqr2<S, G>;
+    auto kern = k_fitter_cqr2<S, G, ALIGNED>;
     const int smem = (int)sizeof(FitterCqr2Shared<S, G>) + 1024;   // + alignment slack
     static std::atomic<bool> allowed[64];
     if (!allowed[dev].load(std::memory_order_relaxed)) {
@@ -445,15 +471,18 @@ static cudaError_t launch_cqr2(int nblocks, int frame, NoiseConst nc, const void
     // three, several teams shorten a block's chain (144 blocks 8.4 us with four
     // teams, 9.8 with two, 12.0 with one; 400 blocks 13.5 with two, 13.9 with
     // one); beyond, one team per block leaves the fewest sums over threads
-    // (1050 blocks 23.8 us against 29.4 with two teams, 3680 blocks 79.6
+    // (1050 blocks 23.8 us against 29.4 with two teams, 3680 blocks 75.2
     // against 87.7).  Four groups of one team fill the registers (255 each).
     const int per_sm = (nblocks + sms - 1) / sms, spread = nblocks < sms ? nblocks : sms;
-    if (fills_with_others(nblocks, beside, sms))
-        return launch_cqr2_t<1, 4>(nblocks, frame, nc, map, weights, mins_maxs, status, dev,
-                                   packed_ctas(nblocks, 4, sms), s);
+    auto one_team = [&](int ctas) {
+        if (nblocks > (kAlignRounds + 2) * 4 * ctas)   // more than six rounds
+            return launch_cqr2_t<1, 4, true>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, ctas, s);
+        return launch_cqr2_t<1, 4>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, ctas, s);
+    };
+    if (fills_with_others(nblocks, beside, sms)) return one_team(packed_ctas(nblocks, 4, sms));
     if (per_sm <= 1) return launch_cqr2_t<4, 1>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
     if (per_sm <= 3) return launch_cqr2_t<2, 3>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
-    return launch_cqr2_t<1, 4>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
+    return one_team(spread);
 }
 
 static cudaError_t launch_rows16(int nblocks, int frame, NoiseConst nc, const void* tmp, float* weights,

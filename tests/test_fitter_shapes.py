@@ -46,6 +46,10 @@ def _draw(rng, blocks, special=True):
     (672, 608),     # 440
     (704, 640),     # 483: four groups per SM
     (1600, 1024),   # 1683: three blocks each
+    (1856, 1280),   # 2419: five
+    (2080, 1440),   # 3036: six
+    (2464, 1440),   # 3588: seven, groups brought together, most idle in the last
+    (2592, 1440),   # 3772: seven
 ])
 def test_cholesky_qr2_shapes_match_fp64(cuda, W, H):
     import torch
