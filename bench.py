@@ -96,19 +96,18 @@ def stage_bytes(w, h):
 
 
 # DRAM bytes (read + write) per launch at 1280x720 from one ncu capture of
-# the kernel (`bench.py --form probe --frames 6 --qr 0`, frame 3's launch;
-# profiles/k_fitter_720p.md, k_taa_720p.md).
-NCU_TRAFFIC_720P = {"fitter": 26.78e6, "taa": 25.94e6}
+# the kernel (`bench.py --form probe --frames 3 --qr 0`, frame 2's launch).
+NCU_TRAFFIC_720P = {"fitter": 26.29e6, "taa": 25.94e6}
 # Warp instructions per launch at 1280x720 (smsp__inst_executed.sum of the
 # same captures): the numerator of the issue-rate roofline of a kernel that
 # is bound by instruction issue rather than by HBM.
-NCU_WARP_INST_720P = {"fitter": 47.24e6, "taa": 11.43e6}
+NCU_WARP_INST_720P = {"fitter": 23.62e6, "taa": 8.82e6}
 SMS, SCHEDULERS_PER_SM = 148, 4
 # Kernels bound by instruction issue rather than by HBM or tensor cores.
 ISSUE_BOUND = {"fitter": "the fitter is a sequence of small dependent reductions and rank-one updates kept "
                          "bit-identical to the reference (no FMA contraction, correctly rounded quotients, binary16 "
-                         "rounding at every store): bound by instruction issue, not by HBM (it reads its 26 MB "
-                         "once) or tensor cores; stages_gbs shows the HBM-bound stages"}
+                         "rounding at every store): bound by instruction issue and the FMA pipe, not by HBM (it reads "
+                         "its 26 MB once) or tensor cores; stages_gbs shows the HBM-bound stages"}
 
 
 MIN_TIMED_SECONDS = 0.5   # each timed region repeats its K-step loop at least this long
@@ -479,9 +478,9 @@ def measure_batched(args, world, rank, local, dev, barrier, steps, warmup):
         "speedup_vs_same_arithmetic_plans": value / prec_value / world,
         "clocks": clocks.summary(),
         # per step: noise table, block kernel, (pixel pass,) TAA (fused); per
-        # stream noise table, accumulation, fitter, weighted sum + filtered
-        # accumulation, TAA (staged)
-        "gpu_launches": (3 + tuning.pixel_pass if pipeline == B.PIPELINE_FUSED else 5 * n) * steps
+        # stream accumulation, fitter, weighted sum + filtered accumulation,
+        # TAA (staged)
+        "gpu_launches": (3 + tuning.pixel_pass if pipeline == B.PIPELINE_FUSED else 4 * n) * steps
                         * len(loop_ms),
     }
 
@@ -893,7 +892,7 @@ def measure_served(args, world, rank, local, dev, barrier, seconds):
                                 "their plans in turn"},
             # per step: 5 kernels per listed stream (staged) or noise, block kernel, (pixel pass,) TAA (fused)
             "clocks": clocks.summary(),
-            "gpu_launches": (5 * int(st.get("frames", 0)) if args.pipeline == "staged"
+            "gpu_launches": (4 * int(st.get("frames", 0)) if args.pipeline == "staged"
                              else (3 + tuning.pixel_pass) * int(st["steps"])),
         }
 
@@ -1054,7 +1053,7 @@ def run_precision(args, world, rank, local, dev, barrier, pg):
                 "psnr_precision_mean": float(np.mean(key("psnr_precision"))),
                 "psnr_fp64_mean": float(np.mean(key("psnr_fp64")))},
             "per_frame": per_frame,
-            "clocks": clocks.summary(), "gpu_launches": 6 * args.steps,
+            "clocks": clocks.summary(), "gpu_launches": 4 * args.steps,
         }), flush=True)
 
 

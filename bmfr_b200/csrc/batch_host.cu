@@ -282,7 +282,7 @@ int fill_desc(bmfr_batch* b, bmfr::BatchStepDesc* d, int n, const int* slots, co
 }
 
 // The staged step on the streams of description d (host copy): for each
-// stream the plan's kernels — noise table, accumulation, fitter, weighted sum
+// stream the plan's kernels — accumulation, fitter, weighted sum
 // + filtered accumulation, TAA — with the stream's buffers, the same
 // launches and arithmetic as a plan's frame, so each stream's output equals
 // the plan's.  The streams are spread over the worker CUDA streams, largest

@@ -329,7 +329,7 @@ int bmfr_plan_keep_intermediates(bmfr_plan* plan, int enable);
  * enabled, every denoise call records CUDA events between its stages.
  * bmfr_plan_stage_times waits for the last frame and returns milliseconds of
  * the staged pipeline's [accumulate_noisy_data (with the frame's fitter
- * noise table), fitter, weighted_sum + accumulate_filtered_data (one kernel
+ * noise table, where the fitter reads one), fitter, weighted_sum + accumulate_filtered_data (one kernel
  * in the plan pipeline), 0, taa].  The fused pipeline reports [noise table,
  * block kernel (accumulate and fitter), weighted_sum +
  * accumulate_filtered_data, 0, taa].  The five drop-in stage entry points
