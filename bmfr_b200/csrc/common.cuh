@@ -128,20 +128,30 @@ __device__ __forceinline__ int floor_index(float v) {
 // Quotients of several numerators by one divisor, each correctly rounded: the
 // divisor's correctly rounded reciprocal and Markstein's correction
 // (q = a*y; r = fma(-q, d, a); q' = fma(r, y, q); negated here, so that zero
-// quotients keep their sign).  `most`: the largest magnitude among the
-// numerators.  A numerator below 2^-100 may round one place off (its residual
-// is no longer exact); every caller adds the quotient to, or compares it with,
-// a value of ordinary size.
+// quotients keep their sign).  That holds where the residual r is exact and
+// the quotient normal: a divisor within 2^+-60 and numerators that are 0 or
+// have magnitudes within [2^-64, 2^60].  `most`: the largest magnitude among
+// the numerators; `least`: the smallest nonzero one, as magnitude_key gives it.
+// NaN numerators pass both tests and are their own quotients.
+//
+// The lower limit is kept because a black pixel's colour is its history alone:
+// a history that fades below 2^-100 otherwise lost its last place to the
+// inexact residual.  It costs an integer operation per numerator.
+__device__ __forceinline__ uint32_t magnitude_key(float a) { return 2u * __float_as_uint(a) - 1u; }   // 0: the largest
 __device__ __forceinline__ bool divides_fast(float d, float most) {
     const float m = fabsf(d);
     return m >= 0x1p-60f && m <= 0x1p60f && most <= 0x1p60f;
+}
+__device__ __forceinline__ bool divides_fast(float d, float most, uint32_t least) {
+    return divides_fast(d, most) && least >= 2u * ((127u - 64u) << 23) - 1u;
 }
 __device__ __forceinline__ float quotient(float a, float ny, float d) {
     const float nq = a * ny;
     return -__fmaf_rn(__fmaf_rn(nq, d, a), ny, nq);
 }
 __device__ __forceinline__ float3 divide3(float3 a, float d) {
-    if (divides_fast(d, fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)))) {
+    const uint32_t least = min(min(magnitude_key(a.x), magnitude_key(a.y)), magnitude_key(a.z));
+    if (divides_fast(d, fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)), least)) {
         const float ny = -__frcp_rn(d);
         return make_float3(quotient(a.x, ny, d), quotient(a.y, ny, d), quotient(a.z, ny, d));
     }

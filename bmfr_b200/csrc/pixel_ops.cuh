@@ -44,6 +44,7 @@ __device__ __forceinline__ AccumResult accumulate_core(
         float uvx = ((m[0] * wp.x + m[4] * wp.y) + m[8] * wp.z) + m[12] * 1.0f;
         float uvy = ((m[1] * wp.x + m[5] * wp.y) + m[9] * wp.z) + m[13] * 1.0f;
         const float w = ((m[3] * wp.x + m[7] * wp.y) + m[11] * wp.z) + m[15] * 1.0f;
+        // No lower limit: 1 is added to these quotients.
         if (divides_fast(w, fmaxf(fabsf(uvx), fabsf(uvy)))) {
             const float ny = -__frcp_rn(w);
             uvx = quotient(uvx, ny, w);
@@ -112,7 +113,10 @@ __device__ __forceinline__ AccumResult accumulate_core(
             total = total + wt[i];
         }
         if (total > 0.0f) {
-            if (divides_fast(total, fmaxf(fmaxf(fabsf(prev.x), fabsf(prev.y)), fmaxf(fabsf(prev.z), sample_spp)))) {
+            const uint32_t least = min(min(magnitude_key(prev.x), magnitude_key(prev.y)),
+                                       min(magnitude_key(prev.z), magnitude_key(sample_spp)));
+            if (divides_fast(total, fmaxf(fmaxf(fabsf(prev.x), fabsf(prev.y)), fmaxf(fabsf(prev.z), sample_spp)),
+                             least)) {
                 const float ny = -__frcp_rn(total);
                 prev.x = quotient(prev.x, ny, total);
                 prev.y = quotient(prev.y, ny, total);
@@ -236,8 +240,7 @@ __device__ __forceinline__ void prepare_block_fit(BlockFit& f, const float* __re
     }
 }
 
-// weighted_sum_px from a prepared block.  A quotient whose numerator is below
-// 2^-100 may round one place off; its product is added to a sum.
+// weighted_sum_px from a prepared block.
 __device__ __forceinline__ float3 weighted_sum_block(float3 wp, float3 n, const BlockFit& b) {
     float v[kFeatures] = {1.0f, n.x, n.y, n.z, wp.x, wp.y, wp.z, wp.x * wp.x, wp.y * wp.y, wp.z * wp.z};
 #pragma unroll
@@ -245,7 +248,7 @@ __device__ __forceinline__ float3 weighted_sum_block(float3 wp, float3 n, const 
         const float a = v[kNotScaled + k] - b.mn[k], d = b.d[k];
         v[kNotScaled + k] = a;
         if (fabsf(d) > 1.0f)   // the same for the whole CTA
-            v[kNotScaled + k] = divides_fast(d, fabsf(a)) ? quotient(a, b.ny[k], d) : a / d;
+            v[kNotScaled + k] = divides_fast(d, fabsf(a), magnitude_key(a)) ? quotient(a, b.ny[k], d) : a / d;
     }
     float3 c = make_float3(0.f, 0.f, 0.f);
 #pragma unroll
