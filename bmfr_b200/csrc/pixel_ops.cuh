@@ -364,12 +364,14 @@ __device__ __forceinline__ void wsacc_px(const Geometry& g, int frame, float sec
 }
 
 // taa body (bmfr.cl:873-973).
-// YCoCg of one colour, unnormalised (bmfr.cl:184-198).  The products by 2 are
-// exact, so each rounds as the reference's multiply and add.
+// YCoCg of one colour, unnormalised (bmfr.cl:184-198).  Products by 2 are
+// sums, which overflow where the reference's products do; the product by 0
+// (NaN for an infinity) is exact and may be fused.
 __device__ __forceinline__ void rgb_to_ycocg(float3 s, float (&ycc)[3]) {
-    ycc[0] = __fmaf_rn(2.0f, s.y, s.x) + s.z;
-    ycc[1] = __fmaf_rn(-2.0f, s.z, __fmaf_rn(0.0f, s.y, s.x + s.x));
-    ycc[2] = __fmaf_rn(2.0f, s.y, -s.x) - s.z;
+    const float x2 = s.x + s.x, y2 = s.y + s.y, z2 = s.z + s.z;
+    ycc[0] = (s.x + y2) + s.z;
+    ycc[1] = __fmaf_rn(0.0f, s.y, x2) - z2;
+    ycc[2] = (y2 - s.x) - s.z;
 }
 
 // The second half of taa (bmfr.cl:904-973) for a pixel whose tonemapped
@@ -418,11 +420,9 @@ __device__ __forceinline__ float3 taa_finish(const Geometry& g, float taa_alpha,
         // A cross without a number has the bounds +inf and -inf.
         if (mnc[c] != mnc[c]) cl[c] = -INFINITY;
     }
-    // The products by 1/4 and 0 are exact (bmfr.cl:965-967).
-    const float a = cl[0] * 0.25f;
-    const float3 rgb = make_float3(__fmaf_rn(-0.25f, cl[2], __fmaf_rn(0.25f, cl[1], a)),
-                                   __fmaf_rn(0.25f, cl[2], __fmaf_rn(0.0f, cl[1], a)),
-                                   __fmaf_rn(-0.25f, cl[2], __fmaf_rn(-0.25f, cl[1], a)));
+    // bmfr.cl:965-967; products by 1/4 round where they are subnormal.
+    const float a = cl[0] * 0.25f, b = cl[1] * 0.25f, c = cl[2] * 0.25f;
+    const float3 rgb = make_float3((a + b) - c, __fmaf_rn(0.0f, cl[1], a) + c, (a - b) - c);
     const float om = 1.0f - taa_alpha;
     return make_float3(taa_alpha * mine.x + om * rgb.x, taa_alpha * mine.y + om * rgb.y,
                        taa_alpha * mine.z + om * rgb.z);

@@ -125,3 +125,23 @@ def test_weighted_sum_of_small_differences(cuda, W, H):
     B.weighted_sum(plan, t(weights), t(mm), got, t(normals), t(positions), None, 3)
     np.testing.assert_array_equal(got.cpu().numpy(), want)
     plan.close()
+
+
+def _taa(cuda, W, H, pix, new, before):
+    import torch
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    plan, o = B.Plan(W, H), Oracle(W, H)
+    want = np.zeros((H, W, 3), np.float32)
+    got = t(want)
+    o.taa(pix, new, want, before, 4)
+    B.taa(plan, t(pix), t(new), got, t(before), 4)
+    np.testing.assert_array_equal(got.cpu().numpy(), want)
+    plan.close()
+
+
+@pytest.mark.parametrize("low,high", [(-149, -120), (118, 127.99)])
+@pytest.mark.parametrize("W,H", [(63, 47), (256, 96)])
+def test_taa_at_the_ends_of_the_range(cuda, W, H, low, high):
+    """Fading histories, products by 2 that overflow, products by 1/4 that round."""
+    rng = np.random.default_rng([W, int(abs(high))])
+    _taa(cuda, W, H, _positions(rng, W, H), _sized(rng, (H, W, 3), low, high), _sized(rng, (H, W, 3), low, high))
