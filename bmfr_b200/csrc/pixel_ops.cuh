@@ -417,8 +417,6 @@ __device__ __forceinline__ float3 taa_finish(const Geometry& g, float taa_alpha,
         const float lo = (mnb[c] + mnc[c]) / 2.0f;
         const float hi = (mxb[c] + mxc[c]) / 2.0f;
         cl[c] = fminf(fmaxf(pyc[c], lo), hi);   // fmin/fmax: the bound where pyc is NaN
-        // A cross without a number has the bounds +inf and -inf.
-        if (mnc[c] != mnc[c]) cl[c] = -INFINITY;
     }
     // bmfr.cl:965-967; products by 1/4 round where they are subnormal.
     const float a = cl[0] * 0.25f, b = cl[1] * 0.25f, c = cl[2] * 0.25f;
@@ -492,6 +490,17 @@ __device__ __forceinline__ void taa_strip(const Geometry& g, int frame, float ta
                         mxb[c] = max3(hmx[up][c], hmx[mid][c], hmx[dn][c]);
                         mnc[c] = min3(own[up][c], hmn[mid][c], own[dn][c]);
                         mxc[c] = max3(own[up][c], hmx[mid][c], own[dn][c]);
+                    }
+                    // A cross, and then perhaps its box, without a number: the
+                    // bounds the reference starts from (bmfr.cl:884-888).
+                    if (mnc[0] != mnc[0] || mnc[1] != mnc[1] || mnc[2] != mnc[2]) {
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            mnb[c] = fminf(mnb[c], INFINITY);
+                            mxb[c] = fmaxf(mxb[c], -INFINITY);
+                            mnc[c] = fminf(mnc[c], INFINITY);
+                            mxc[c] = fmaxf(mxc[c], -INFINITY);
+                        }
                     }
                     out = taa_finish(g, taa_alpha, pp, ix, iy, mine, mnb, mxb, mnc, mxc, prev_frame);
                 }

@@ -145,3 +145,19 @@ def test_taa_at_the_ends_of_the_range(cuda, W, H, low, high):
     """Fading histories, products by 2 that overflow, products by 1/4 that round."""
     rng = np.random.default_rng([W, int(abs(high))])
     _taa(cuda, W, H, _positions(rng, W, H), _sized(rng, (H, W, 3), low, high), _sized(rng, (H, W, 3), low, high))
+
+
+@pytest.mark.parametrize("W,H", [(63, 47), (256, 96)])
+def test_taa_cross_without_a_number(cuda, W, H):
+    """A cross without a number has the bounds +inf and -inf, whatever its
+    box's corners hold: numbers, infinities, NaN.  One NaN channel makes the
+    cross NaN and leaves the pixel's others to be seen."""
+    rng = np.random.default_rng(W)
+    new, before = _sized(rng, (H, W, 3), -3, 3, 0.0), _sized(rng, (H, W, 3), -3, 3, 0.05)
+    for y in range(1, H - 1, 3):
+        for x in range(1, W - 1, 3):
+            ch = rng.integers(0, 3)
+            new[y, x - 1:x + 2, ch], new[y - 1:y + 2, x, ch] = np.nan, np.nan
+            for dy, dx in ((-1, -1), (-1, 1), (1, -1), (1, 1)):
+                new[y + dy, x + dx] = rng.choice([0.5, 2.0, np.inf, -np.inf, np.nan])
+    _taa(cuda, W, H, _positions(rng, W, H), new, before)
