@@ -107,16 +107,6 @@ __device__ __forceinline__ void await_previous_kernel() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// convert_int_rtn with defined results: NaN and magnitudes beyond 2^30 map to
-// +-2^30, outside every image.
-__device__ __forceinline__ int floor_to_int(float v) {
-    if (!(v == v)) return -(1 << 30);
-    const float f = floorf(v);
-    if (f < -1073741824.0f) return -(1 << 30);
-    if (f > 1073741824.0f) return 1 << 30;
-    return (int)f;
-}
-
 // convert_int_rtn for indices that are tested against an image before use:
 // saturates, and NaN maps to INT_MIN.  i and i + 1 (in unsigned arithmetic)
 // lie outside every image wherever the position does.
@@ -169,21 +159,6 @@ __device__ __forceinline__ float hash_random(uint32_t a) {
     return __uint2float_rn(a) / 4294967296.0f;   // convert_float(UINT_MAX) = 2^32
 }
 
-// add_random (bmfr.cl:173-182): value + NOISE_AMOUNT*2*(random(i) - 0.5),
-// rounded once to float.  The product c*r (c = hi + lo) is formed exactly
-// enough with fma error terms (Dekker/Ogita-Rump-Oishi two-product and
-// two-sum), then the three-term sum is rounded once.
-__device__ __forceinline__ float add_noise(float value, uint32_t index, NoiseConst c) {
-    const float r = hash_random(index) - 0.5f;
-    const float p = c.hi * r;
-    const float pe = __fmaf_rn(c.hi, r, -p);          // exact error of c.hi*r
-    const float pl = __fmaf_rn(c.lo, r, pe);          // + c.lo*r
-    const float s = value + p;                        // two-sum(value, p)
-    const float bv = s - value;
-    const float se = (value - (s - bv)) + (p - bv);
-    return s + (se + pl);
-}
-
 __device__ __forceinline__ uint32_t noise_index(int id, int sub_vector, int feature, int frame) {
     return (uint32_t)id + (uint32_t)sub_vector * (uint32_t)kLocal +
            (uint32_t)feature * (uint32_t)kBlockPixels +
@@ -208,17 +183,6 @@ __device__ __forceinline__ __half2 pack_features(float a, float b) {
     const __half2 h = *reinterpret_cast<__half2*>(&v);
     v &= __heq2_mask(h, h);
     return *reinterpret_cast<__half2*>(&v);
-}
-
-// Store of one tmp_data value, binary16 or float32 (bmfr.cl:255-265, 468-475).
-__device__ __forceinline__ void store_feature(void* tmp, size_t i, float v, bool half_tmp) {
-    if (v != v) v = 0.0f;
-    if (half_tmp) {
-        v = fmaxf(fminf(v, 65504.0f), -65504.0f);
-        reinterpret_cast<__half*>(tmp)[i] = __float2half_rn(v);
-    } else {
-        reinterpret_cast<float*>(tmp)[i] = v;
-    }
 }
 
 __device__ __forceinline__ void hist_store(float* p, int i, float3 v) {

@@ -191,18 +191,6 @@ struct Tile<false> {   // float storage: no intermediate rounding; rows (q0,q1) 
     }
 };
 
-// value + NOISE_AMOUNT*2*r with r = random(i) - 0.5 already formed
-// (bmfr.cl:173-182), rounded once (see add_noise in common.cuh).
-__device__ __forceinline__ float add_noise_r(float value, float r, NoiseConst c) {
-    const float p = c.hi * r;
-    const float pe = __fmaf_rn(c.hi, r, -p);
-    const float pl = __fmaf_rn(c.lo, r, pe);
-    const float s = value + p;
-    const float bv = s - value;
-    const float se = (value - (s - bv)) + (p - bv);
-    return s + (se + pl);
-}
-
 // True division, kept out of line so that the rare slow case costs no code
 // at every call site.
 static __device__ __noinline__ float div_slow(float a, float b) { return a / b; }
@@ -274,7 +262,10 @@ __device__ __forceinline__ float add_f32_h(__half a, float c) {
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 
-// add_noise_r on two values at once.
+// add_random (bmfr.cl:173-182) on two values at once: value + NOISE_AMOUNT*2*r,
+// r = random(i) - 0.5 already formed, rounded once.  The product c*r (c = hi +
+// lo) is formed exactly enough with fma error terms (Dekker/Ogita-Rump-Oishi
+// two-product and two-sum), then the three-term sum is rounded once.
 __device__ __forceinline__ float2 add_noise_r2(float2 v, float2 r, NoiseConst c) {
     const float2 hi = dup2(c.hi), lo = dup2(c.lo);
     const float2 p = rmul2(hi, r, c.neg_zero);
@@ -790,8 +781,8 @@ __device__ __forceinline__ void gram_finish(FitterSmem& sm) {
 // the Gram matrix (g[i], i <= j; zeros below) and stores its diagonal entry
 // in diag[j]; lanes 10..12 gather the colour column c = lane - 10 of the
 // second pass; other lanes zeros.
-template <bool PASS2, typename Smem>
-__device__ __forceinline__ void gram_columns(Smem& sm, int lane, float (&g)[kFeatures]) {
+template <bool PASS2>
+__device__ __forceinline__ void gram_columns(FitterSmem& sm, int lane, float (&g)[kFeatures]) {
 #pragma unroll
     for (int i = 0; i < kFeatures; ++i) {
         int e = -1;

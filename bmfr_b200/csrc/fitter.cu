@@ -51,13 +51,6 @@ struct FitterShared {
     float noise[NOISE_GLOBAL ? 1 : kNoiseTableFloats];
 };
 
-// Byte offset of half h of a block tile copied with the 128-byte swizzle:
-// row h / 64, 16-byte chunk (h % 64) / 8 XOR the row's low three bits.
-__device__ __forceinline__ uint32_t swizzled_half(uint32_t h) {
-    const uint32_t r = h >> 6, c = h & 63u;
-    return (r << 7) | ((((c >> 3) ^ r) & 7u) << 4) | ((c & 7u) << 1);
-}
-
 // METHOD (FitMethod): the FP32 Householder sequence on binary16 tmp_data, or
 // the reference's arithmetic on float tmp_data, which rounds nowhere in
 // between; both work on a float tile.
@@ -115,7 +108,7 @@ __global__ void __launch_bounds__(256, 2)
         // (low three row bits) does not depend on k.
         uint32_t qoff[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) qoff[q] = swizzled_half((uint32_t)(q * kLocal + id));
+        for (int q = 0; q < 4; ++q) qoff[q] = swizzled_in_column((uint32_t)(q * kLocal + id));
 #pragma unroll
         for (int k = 0; k < kBuffers; ++k) {
             if constexpr (HALF_TMP) {

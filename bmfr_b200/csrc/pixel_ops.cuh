@@ -159,7 +159,8 @@ __device__ __forceinline__ void store_tmp_row(const Geometry& g, void* tmp, bool
         }
     } else {
 #pragma unroll
-        for (int k = 0; k < kBuffers; ++k) store_feature(tmp, base + (size_t)k * kBlockPixels, f[k], false);
+        for (int k = 0; k < kBuffers; ++k)
+            static_cast<float*>(tmp)[base + (size_t)k * kBlockPixels] = f[k] != f[k] ? 0.0f : f[k];
     }
 }
 
