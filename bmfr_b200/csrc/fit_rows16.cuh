@@ -30,7 +30,6 @@
 namespace bmfr {
 
 constexpr int kTeam = 64;         // threads of a team
-constexpr int kWide = 2;          // later columns in flight per thread
 constexpr int kRowPairs = 8;      // row pairs per thread: rows i + 128*p and i + 128*p + 64
 // 16-byte chunks of the tile: [column][chunk][thread]; raw tmp_data at first.
 constexpr int kTileChunks = kBuffers * 2 * kTeam;
@@ -307,6 +306,10 @@ __device__ __forceinline__ void qr_column16(int col, int i, int team, Reflection
         }
     };
     const int end = MODE == 0 ? 9 : kBuffers;   // column 0 alone has room for eight values
+    // Later columns in flight per thread.  Teams that share a block overlap
+    // each other's chains, and with one column at a time their CTAs fit in 128
+    // registers (two at a time there: 294 blocks 21.7 us against 20.9).
+    constexpr int kWide = S == 1 ? 2 : 1;
     int k = col + 1 + team;
 #pragma unroll 1
     for (; k + (kWide - 1) * S < end; k += kWide * S) visit(std::integral_constant<int, kWide>{}, k);

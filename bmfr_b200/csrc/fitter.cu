@@ -152,8 +152,20 @@ struct FitterRows16Shared {
     alignas(16) float noise[kNoiseTableFloats];
 };
 
+// CTAs per SM.  A launch does not know what runs beside it: a caller may have
+// plans on streams of its own.  With up to two blocks per SM a CTA therefore
+// takes at most half of an SM, so that the fits of two streams share it.  Eight
+// plans on eight streams, us per round of frames, with CTAs of a whole SM / of
+// half / with one thread per work-item: 320x240 127 / 92 / 97, 400x340 201 / 135
+// / 163, 640x360 271 / 207 / 263.  Alone, 99 blocks take 16.4 instead of 16.2
+// us, 273 blocks 20.8 instead of 20.7.
 template <int S, int G>
-__global__ void __launch_bounds__(kTeam * S * G, 1)
+constexpr int kRows16Ctas = G == 1 || G == 2 ? 2 : 1;
+constexpr int kSmemPerSm = 228 * 1024, kSmemPerCta = 2048;   // capacity; a CTA's alignment slack and reserve
+static_assert(2 * (sizeof(FitterRows16Shared<2>) + kSmemPerCta) <= kSmemPerSm, "two CTAs of two groups share an SM");
+
+template <int S, int G>
+__global__ void __launch_bounds__(kTeam * S * G, kRows16Ctas<S, G>)
     k_fitter_rows16(int nblocks, int frame, NoiseConst nc, const __grid_constant__ CUtensorMap tmap,
                     float* __restrict__ weights, float* __restrict__ mins_maxs, int* __restrict__ status) {
     using Shared = FitterRows16Shared<G>;
@@ -229,8 +241,15 @@ struct FitterCqr2Shared {
     alignas(16) float noise[kNoiseTableFloats];
 };
 
+// CTAs per SM, as for k_fitter_rows16; eight plans on eight streams: 320x240 76 /
+// 69 / 68, 400x340 138 / 114 / 115, 640x360 189 / 171 / 185.  Alone, 99 blocks
+// stay at 8.0 us and 273 blocks take 11.9 instead of 11.0.
+template <int S, int G>
+constexpr int kCqr2Ctas = G == 1 || G == 2 ? 2 : 1;
+static_assert(2 * (sizeof(FitterCqr2Shared<2, 2>) + kSmemPerCta) <= kSmemPerSm, "two CTAs of two groups share an SM");
+
 template <int S, int G, bool ALIGNED>
-__global__ void __launch_bounds__(kTeam * S * G, 1)
+__global__ void __launch_bounds__(kTeam * S * G, kCqr2Ctas<S, G>)
     k_fitter_cqr2(int nblocks, int frame, NoiseConst nc, const __grid_constant__ CUtensorMap tmap,
                   float* __restrict__ weights, float* __restrict__ mins_maxs, int* __restrict__ status) {
     using Shared = FitterCqr2Shared<S, G>;
@@ -268,10 +287,11 @@ __global__ void __launch_bounds__(kTeam * S * G, 1)
             }
             return false;
         }
-        fit_cqr2<S>(reinterpret_cast<const unsigned char*>(tile), reinterpret_cast<const float4*>(sh.noise), nc.hi, t,
-                    sm, bar, weights + (size_t)b * kFeatures * 3, mins_maxs + (size_t)b * kScaled * 2, [&] {
-                        if (leader && b + stride < nblocks) issue(b + stride);
-                    });
+        fit_cqr2<S, S == 2 && kCqr2Ctas<S, G> == 2>(
+            reinterpret_cast<const unsigned char*>(tile), reinterpret_cast<const float4*>(sh.noise), nc.hi, t, sm, bar,
+            weights + (size_t)b * kFeatures * 3, mins_maxs + (size_t)b * kScaled * 2, [&] {
+                if (leader && b + stride < nblocks) issue(b + stride);
+            });
         return true;
     };
     if constexpr (ALIGNED) {
@@ -474,6 +494,7 @@ static cudaError_t launch_cqr2(int nblocks, int frame, NoiseConst nc, const void
     };
     if (fills_with_others(nblocks, beside, sms)) return one_team(packed_ctas(nblocks, 4, sms));
     if (per_sm <= 1) return launch_cqr2_t<4, 1>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
+    if (per_sm <= 2) return launch_cqr2_t<2, 2>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
     if (per_sm <= 3) return launch_cqr2_t<2, 3>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
     return one_team(spread);
 }
@@ -504,6 +525,7 @@ static cudaError_t launch_rows16(int nblocks, int frame, NoiseConst nc, const vo
         return launch_rows16_t<1, 6>(nblocks, frame, nc, map, weights, mins_maxs, status, dev,
                                      packed_ctas(nblocks, 6, sms), s);
     if (per_sm <= 1) return launch_rows16_t<4, 1>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
+    if (per_sm <= 2) return launch_rows16_t<2, 2>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
     if (per_sm <= 3) return launch_rows16_t<2, 3>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
     if (per_sm <= 21 && (per_sm + 6) / 7 < (per_sm + 5) / 6)
         return launch_rows16_t<1, 7>(nblocks, frame, nc, map, weights, mins_maxs, status, dev, spread, s);
