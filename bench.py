@@ -99,15 +99,15 @@ def stage_bytes(w, h):
 # the kernel (`bench.py --form probe --frames 3 --qr 0`, frame 2's launch).
 NCU_TRAFFIC_720P = {"fitter": 26.29e6, "taa": 25.94e6}
 # Warp instructions per launch at 1280x720 (smsp__inst_executed.sum of the
-# same captures): the numerator of the issue-rate roofline of a kernel that
-# is bound by instruction issue rather than by HBM.
-NCU_WARP_INST_720P = {"fitter": 23.62e6, "taa": 8.82e6}
+# same captures): the numerator of the issue-rate roofline of a kernel whose
+# instruction stream, not HBM, sets its time.
+NCU_WARP_INST_720P = {"fitter": 23.62e6, "taa": 9.25e6}
 SMS, SCHEDULERS_PER_SM = 148, 4
-# Kernels bound by instruction issue rather than by HBM or tensor cores.
+# Kernels bound by their instruction stream rather than by HBM or tensor cores.
 ISSUE_BOUND = {"fitter": "the fitter is a sequence of small dependent reductions and rank-one updates kept "
                          "bit-identical to the reference (no FMA contraction, correctly rounded quotients, binary16 "
-                         "rounding at every store): bound by instruction issue and the FMA pipe, not by HBM (it reads "
-                         "its 26 MB once) or tensor cores; stages_gbs shows the HBM-bound stages"}
+                         "rounding at every store): bound by the latency of its dependent steps, with issue slots and "
+                         "the FMA-heavy pipe about half used, not by HBM (it reads its 26 MB once) or tensor cores"}
 
 
 MIN_TIMED_SECONDS = 0.5   # each timed region repeats its K-step loop at least this long
@@ -890,7 +890,7 @@ def measure_served(args, world, rank, local, dev, barrier, seconds):
                                 "step per frame of all streams (staged: each stream's plan kernels on eight "
                                 "worker CUDA streams; fused: one graph-captured block-queue launch); plain: "
                                 "their plans in turn"},
-            # per step: 5 kernels per listed stream (staged) or noise, block kernel, (pixel pass,) TAA (fused)
+            # per step: 4 kernels per listed stream (staged) or noise, block kernel, (pixel pass,) TAA (fused)
             "clocks": clocks.summary(),
             "gpu_launches": (4 * int(st.get("frames", 0)) if args.pipeline == "staged"
                              else (3 + tuning.pixel_pass) * int(st["steps"])),
@@ -1265,7 +1265,7 @@ def main():
         "frame_loop": other_loop, "value": world * args.steps / (other_loop_ms / 1e3), "unit": "frames/s",
         "ms_per_step": other_loop_ms / args.steps,
         "how": "sequence: the K frames of a loop in one bmfr_denoise_frames call, each frame's accumulation "
-               "overlapping the previous frame's fitter, weighted sum and TAA (same outputs bit for bit); "
+               "overlapping the previous frame's weighted sum and TAA (same outputs bit for bit); "
                "single: one bmfr_denoise_frame_io call per frame, stages in stream order"}
     # noise table, block kernel, weighted sum + filtered accumulation, taa
     # (fused); accumulate, fitter, weighted sum + filtered accumulation, taa

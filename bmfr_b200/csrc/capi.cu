@@ -711,10 +711,10 @@ int bmfr_denoise_frames(bmfr_plan* plan, int count, const bmfr_frame_io* io, con
                 return cuda_fail(e, "denoise_frames: frame order");
             }
         }
-        // A fitter that keeps every SM busy leaves the accumulation nothing to
-        // run on but SMs that the fitter then starts late on, so there the
+        // A fitter that takes every SM leaves the accumulation nothing to run
+        // on but SMs that the fitter then starts late on, so there the
         // accumulation waits for frame f-1's fit and overlaps the stages
-        // behind it.
+        // behind it (fitter_fills_gpu has both sides measured).
         if (overlap && i >= 1 && fit_first) {
             cudaError_t e = cudaStreamWaitEvent(sa, plan->ev_fitted, 0);
             if (e != cudaSuccess) {

@@ -7,8 +7,8 @@
 // reference's reduction tree (bmfr.cl:32-33), so that stage runs on the
 // thread's own values, and everything a thread does once per column (the
 // norm's last stages, the square root, the reciprocal, the loop) is done by
-// 2*S warps instead of the eight that one thread per work-item takes.  The
-// fit is bound by instruction issue: see the measurements at k_fitter_rows16.
+// 2*S warps instead of the eight that one thread per work-item takes.  What
+// bounds it, and what that gave, stands at k_fitter_rows16.
 //
 // The columns lie in shared memory as binary16, rounded at every in-place
 // store as the reference's tmp_data is, a thread's 16 rows of a column in two
@@ -220,8 +220,9 @@ __device__ __forceinline__ Rows update_rows(const Rows& x, int k, int i, const R
 // applies the first column's update to the noised features; 2: the others.
 // PLAIN: column 0 is all ones and the noise below 1, as in every frame the
 // pipeline makes; the other instance serves callers' own tmp_data and noise
-// (a test of the noise inside the loops cost 12 % of the time).  f: the previous column's reflection on entry,
-// this one's on return; out holds the dot products that go with it.
+// (a test of the noise inside the loops cost 12 % of the time).  f: the
+// previous column's reflection on entry, this one's on return; out holds the
+// dot products that go with it.
 template <int S, int MODE, bool PLAIN>
 __device__ __forceinline__ void qr_column16(int col, int i, int team, Reflection& f, const float4* __restrict__ noise,
                                             NoiseConst nc, Rows16Smem& sm, uint4* tile, int bar) {

@@ -137,11 +137,12 @@ __global__ void __launch_bounds__(256, 2)
 // The CTA forms the frame's noise table in its shared memory, which its groups
 // share; that saves the launch that wrote it to global memory (2.0-2.4 us).
 //
-// Bound by the FMA pipes: a packed operation takes two cycles on one of them
-// and a scalar one the same slot on either, ~21 k such cycles per warp and
-// block, of which a column's rank-one updates are half.  From four groups on
-// an SM the time hardly falls with more of them (8349 blocks: 365 us with
-// four, 318 with five, 295 with six).  One thread per work-item, 256 threads
+// Bound by the dependent steps of each column (norm, square root, dot products,
+// update), with FMA and issue slots about half used: 984 blocks issue on 54 %
+// of the cycles with the FMA-heavy pipe 45 % active, 8349 blocks on 55 % with
+// it 53 % active, and the longest stall is the fixed latency of the operation
+// before (1.4 cycles per issue).  More groups on an SM fill the gaps (8349
+// blocks: 365 us with four, 318 with five, 295 with six).  One thread per work-item, 256 threads
 // per block and the columns in registers took 47 M warp instructions for the
 // 984 blocks of 1280x720, this takes 23 M: 69.5 -> 42.5 us; 2135 blocks
 // (1920x1080) 148 -> 87 us; 8349 (3840x2160) 543 -> 295 us.
@@ -216,15 +217,15 @@ __global__ void __launch_bounds__(kTeam * S * G, kRows16Ctas<S, G>)
 // The precision form's CholeskyQR2 fit (fit_cqr2.cuh): G groups of S teams per
 // CTA, one CTA per SM, as k_fitter_rows16.
 //
-// Bound by the FMA pipes (~2.4 k cycles of each scheduler per block: the
-// Gram entries' multiplies, fused multiply-adds and sums in the kept order)
-// and, with four blocks in flight, the two factorisations between and behind
-// the passes.  256 threads per block took, against this: 135 blocks 11.7 -> 8.3
+// Bound by latency at two warps per scheduler, which is what the registers
+// allow: 984 blocks issue on 32 % of the cycles with the FMA-heavy pipe 29 %
+// active (stalls per issue: instruction fetch 1.5, the operation before 1.1,
+// barriers around warp 0's two factorisations 0.7), 8349 blocks on 44 % with it
+// 46 % active.  256 threads per block took, against this: 135 blocks 11.7 -> 8.3
 // us, 984 (1280x720) 37 -> 23.7, 2135 (1920x1080) 72 -> 44, 8349 (3840x2160)
 // 252 -> 152 us.
 //
-// The fit is straight-line code that each group passes once per block, and
-// waiting for instructions is its longest stall (1.3 cycles per issue).  Groups
+// The fit is straight-line code that each group passes once per block.  Groups
 // that have drifted apart fetch it four times over, so from the seventh round
 // on it pays to bring them back together (ALIGNED: a barrier of the CTA every
 // fourth round): 3680 blocks 79.0 -> 75.2 us, 4736 101 -> 90.5, 8228 179 -> 153
@@ -463,6 +464,14 @@ static cudaError_t device_sms(int* dev, int* sms) {
 // others.  A step of eight 640x360 streams took 349 us spread and 294 packed
 // with CholeskyQR2, 503 and 370 with the reference's arithmetic; five streams
 // of 380 blocks together 184 spread and 193 packed.
+//
+// A packed launch of the reference's arithmetic takes six groups per CTA where
+// a launch alone might take seven.  Beside smaller or larger streams that is
+// the faster one, beside streams of its own size the slower one (steps of
+// 1280x720 with others, us with six / seven: 64x48 128 / 134, 320x240 129 /
+// 133, 1920x1080 297 / 311, 3840x2160 808 / 857; one, two or seven of the same
+// size 205 / 190, 303 / 283, 796 / 744; 853x481 158 / 149); `beside` does not
+// tell them apart.
 static bool fills_with_others(int nblocks, int beside, int sms) { return beside > 0 && nblocks + beside > 4 * sms; }
 
 // CTAs of `groups` groups that `nblocks` blocks fill, at most one per SM.

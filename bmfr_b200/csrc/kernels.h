@@ -50,11 +50,15 @@ cudaError_t launch_fitter(const Geometry& g, int frame, NoiseConst nc, const voi
                           int qr, float* weights, float* mins_maxs, const float* noise_table, int* status,
                           cudaStream_t s, int beside = 0);
 cudaError_t launch_noise_table(int frame, float* table, cudaStream_t s);
-// Whether work beside launch_fitter's kernel only delays it: measured with the
-// next frame's accumulation beside it, us per frame against none: reference
+// Whether a clip's next accumulation starts behind launch_fitter's kernel
+// instead of beside it.  Measured beside / behind, us per frame: reference
 // arithmetic on binary16 tmp_data 1920x1080 203.7 / 197.9, 3840x2160 735.6 /
 // 692.7; CholeskyQR2 149.2 / 156.2, 547 / 565; float tmp_data 1280x720 126.1 /
-// 136.1.
+// 136.1.  Smaller images change by little with the reference's arithmetic,
+// either way (us per clip of eight or six: 64x48 199 / 205, 320x240 217 / 215,
+// 640x360 299 / 301, 1024x576 529 / 553, 1120x630 462 / 451, 1216x704 528 /
+// 553, 1280x720 764 / 768, 1312x768 677 / 659, 1600x900 872 / 857), so the rule
+// has no size in it.
 bool fitter_fills_gpu(bool half_tmp, int qr);
 // Whether launch_fitter reads `noise_table`, so that a frame has to make it.
 bool fitter_reads_noise_table(bool half_tmp, int qr);

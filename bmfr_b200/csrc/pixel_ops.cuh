@@ -449,8 +449,7 @@ __device__ __forceinline__ void taa_strip(const Geometry& g, int frame, float ta
     float3 rgb[3];
     float own[3][3], hmn[3][3], hmx[3][3];   // [window row][channel]
     // The strip's reprojected positions first: the history gather of each
-    // row depends on them, and they depend on nothing here (1920x1080
-    // frame 319.4 -> 315.2 us).
+    // row depends on them, and they depend on nothing here.
     float2 ppre[R];
 #pragma unroll
     for (int rr = 0; rr < R; ++rr) {

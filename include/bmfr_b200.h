@@ -284,9 +284,9 @@ int bmfr_denoise_frame_io(bmfr_plan* plan, const bmfr_frame_io* io,
  * accumulated history, and the plan alternates two sets of the per-frame
  * buffers it writes (tmp_data, reprojected positions, accept mask, fitter
  * noise table).  The first such call allocates that second set (about 37 B
- * per pixel with binary16 tmp_data).  Where the fitter keeps every SM busy (the
- * reference's arithmetic on binary16 tmp_data), that accumulation starts behind
- * frame i's fitter.  The buffers io[] points to must not be written while the
+ * per pixel with binary16 tmp_data).  With the reference's arithmetic on
+ * binary16 tmp_data that accumulation starts behind frame i's fitter, at every
+ * image size.  The buffers io[] points to must not be written while the
  * call's work runs.  The fused pipeline, and any call while stage profiling
  * is on, runs the frames one after another on `stream`.  Every frame's
  * arguments are checked before the first is queued; a CUDA error part way
