@@ -362,9 +362,12 @@ __device__ __forceinline__ void qr_column(Tile<HALF>& t, int col, int id, const 
     if (id == col) sm.Rm[col][col] = vl;
     const float u0 = id == col ? ucl_new : c01.x;
     const bool row0 = id >= col;
-    // Rows below the column (only row id can be) take no part in the dot:
-    // 0 + a*0 leaves the reference's partial sum 0 unchanged.
-    const float2 uq0 = dup2(row0 ? u0 : 0.0f), uq1 = dup2(c01.y), uq2 = dup2(c23.x), uq3 = dup2(c23.y);
+    // Rows above the column (only row id can be) take no part in the dot: with
+    // float columns 0 + a*0 leaves the reference's partial sum 0 unchanged (an
+    // infinite a lies in a column that is not finite anywhere); a binary16
+    // column may have overflowed in that row alone, and its sum starts at 0
+    // behind it.
+    const float2 uq0 = dup2(HALF || row0 ? u0 : 0.0f), uq1 = dup2(c01.y), uq2 = dup2(c23.x), uq3 = dup2(c23.y);
 
     // Dot products with the later columns (bmfr.cl:606-638): 0 + p0 + p1 +
     // p2 + p3 in the reference's order for rows q0..q3.
@@ -386,6 +389,10 @@ __device__ __forceinline__ void qr_column(Tile<HALF>& t, int col, int id, const 
                 d[i] = s.x;
                 d[i + 1] = s.y;
             }
+        }
+        if (8 * (int)(threadIdx.x >> 5) < col) {   // the first two warps alone hold such rows
+#pragma unroll
+            for (int i = 0; i < VS; ++i) d[i] = row0 ? d[i] : 0.0f;
         }
         // Rows q1..q3: a binary16 product is exact in float, so s + a*u
         // rounds once either way and is one mixed-precision FMA.
