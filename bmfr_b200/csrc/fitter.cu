@@ -133,7 +133,8 @@ __global__ void __launch_bounds__(256, 2)
 }
 
 // The reference-arithmetic fit of binary16 tmp_data (fit_rows16.cuh): G groups
-// of S teams per CTA, one CTA per SM, each group walking blocks of its own.
+// of S teams per CTA, one CTA per SM or two (kRows16Ctas), each group walking
+// blocks of its own.
 // The CTA forms the frame's noise table in its shared memory, which its groups
 // share; that saves the launch that wrote it to global memory (2.0-2.4 us).
 //
@@ -142,10 +143,10 @@ __global__ void __launch_bounds__(256, 2)
 // of the cycles with the FMA-heavy pipe 45 % active, 8349 blocks on 55 % with
 // it 53 % active, and the longest stall is the fixed latency of the operation
 // before (1.4 cycles per issue).  More groups on an SM fill the gaps (8349
-// blocks: 365 us with four, 318 with five, 295 with six).  One thread per work-item, 256 threads
-// per block and the columns in registers took 47 M warp instructions for the
-// 984 blocks of 1280x720, this takes 23 M: 69.5 -> 42.5 us; 2135 blocks
-// (1920x1080) 148 -> 87 us; 8349 (3840x2160) 543 -> 295 us.
+// blocks: 365 us with four, 318 with five, 295 with six).  One thread per
+// work-item, 256 threads per block and the columns in registers, took 47 M warp
+// instructions for the 984 blocks of 1280x720, this takes 23 M: 69.5 -> 42.2 us;
+// 2135 blocks (1920x1080) 148 -> 87 us; 8349 (3840x2160) 543 -> 294 us.
 template <int G>
 struct FitterRows16Shared {
     uint4 tile[G][kTileChunks];   // 1024-byte aligned, for the swizzled copy
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(kTeam * S * G, kRows16Ctas<S, G>)
 }
 
 // The precision form's CholeskyQR2 fit (fit_cqr2.cuh): G groups of S teams per
-// CTA, one CTA per SM, as k_fitter_rows16.
+// CTA, one CTA per SM or two (kCqr2Ctas), as k_fitter_rows16.
 //
 // Bound by latency at two warps per scheduler, which is what the registers
 // allow: 984 blocks issue on 32 % of the cycles with the FMA-heavy pipe 29 %
